@@ -9,7 +9,7 @@ DataGenerator ("uniform" over [0, 2^32), seed 2147483647). Per rank:
           its CUDA-event timed region; inputs (4 GiB) exceed L2 (126 MB).
   e2e   : keys/s of mgs_sort_host (TanasicSort with one GPU: pinned host
           buffer, H2D + sort + D2H inside the timed call), wall-clock.
-  roofline: the onesweep pass kernel, algorithmic bytes (read + write of the
+  roofline: the scatter kernel of the partition sort, algorithmic bytes (read + write of the
           keys) per launch over its CUDA-event time, against the measured HBM
           copy bandwidth.
   cpu_baseline: the reference's CPU sort (the gnu_parallel branch of
@@ -67,7 +67,7 @@ def measured_hbm_peak():
 
 def committed_traffic(kernel: str):
     """DRAM bytes per launch of `kernel` from the committed ncu summary, if any."""
-    p = os.path.join(ROOT, "profiles", "radix_onesweep_u32.md")
+    p = os.path.join(ROOT, "profiles", f"{kernel}_u32.md")
     if not os.path.exists(p):
         return None
     for line in open(p):
@@ -1061,18 +1061,17 @@ def main():
     e2e_value = job_keys_per_s(world, n, len(e2e_times), e2e_s) if e2e_times else None
 
     peak, peak_kind = measured_hbm_peak()
-    one = ktimes.get("radix_onesweep", (0, 0.0))
-    hist = ktimes.get("radix_histogram", (0, 0.0))
+    one = ktimes.get("part_scatter", (0, 0.0))
     roof = None
     if one[0] > 0:
         avg_ms = one[1] / one[0]
-        alg_bytes = 2 * 4 * n  # each pass reads and writes every key
+        alg_bytes = 2 * 4 * n  # each scatter reads and writes every key
         achieved = alg_bytes / (avg_ms / 1e3) / 1e9
-        traffic = committed_traffic("radix_onesweep") if n == N_KEYS else None
-        roof = {"bound": "hbm", "kernel": "radix_onesweep", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        traffic = committed_traffic("part_scatter") if n == N_KEYS else None
+        roof = {"bound": "hbm", "kernel": "part_scatter", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
                 "traffic": traffic, "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms}
-    sort_alg_bytes = 36 * n  # 4 passes x (read + write) + one histogram read, 4-byte keys
+    sort_alg_bytes = 36 * n  # a radix sort's 4 passes x (read + write) + one histogram read, 4-byte keys
     sort_ms = total_ms / args.steps
 
     batched = None

@@ -100,7 +100,8 @@ int mgs_host_free(void* ptr);
  * Ascending, stable, in place on d_keys. d_temp must hold mgs_sort_temp_bytes()
  * bytes, or be NULL to use the context arena. stream is a cudaStream_t (NULL =
  * the context's compute stream). Asynchronous: device status is reported by
- * mgs_ctx_synchronize. n must be below 2^32. */
+ * mgs_ctx_synchronize. n must be below 2^32. Runs a partition sort, unless
+ * mgs_tune_set (or its environment variables) asked for an onesweep variant. */
 int mgs_sort_temp_bytes(int dtype, size_t n, size_t* bytes);
 int mgs_sort_device(mgs_ctx* ctx, int dtype, void* d_keys, size_t n, void* d_temp, size_t temp_bytes,
                     void* stream);
@@ -231,13 +232,16 @@ int mgs_plan_destroy(mgs_plan* plan); /* waits for the device first (replays may
 
 /* ---- onesweep variants and the autotuner ------------------------------------
  * No counterpart in the reference (it calls thrust::sort with CUB's own tuning).
- * The radix sort picks, per key width (4 or 8 bytes) and size class of n
+ * The onesweep radix sort picks, per key width (4 or 8 bytes) and size class of n
  * (0: n < 2^16, 1: < 2^18, 2: < 2^20, 3: < 2^22, 4: < 2^26, 5: larger), a tile
  * shape (0..6: threads x keys per thread) and a ranking mode (2: shared-memory
  * peer masks, 3: ballots for half of the keys). The table is read from a tuning
  * file on first use (MGS_TUNE_FILE, else tuning/b200.tune beside the library's
  * directory; format: lines "key_bytes size_class shape rank_mode"), and the
  * environment variables MGS_ONESWEEP_SHAPE / MGS_RANK_MODE override it.
+ * Plain sorts run the onesweep only for classes set through mgs_tune_set (until
+ * the next mgs_tune_load or mgs_autotune) or under those variables; otherwise
+ * they are partition sorts, which are faster.
  * mgs_autotune times every variant on a sample of each size class up to max_n
  * (uniformly random keys of the dtype's width, median of reps sorts), keeps the
  * fastest in the table and reports every timing in out (count = number of

@@ -746,7 +746,7 @@ int mgs_tune_get(int dtype, size_t n, int* shape, int* rank_mode) {
 int mgs_tune_set(int dtype, int size_class, int shape, int rank_mode) {
   const size_t w = mgs::dtype_bytes(dtype);
   if (w == 0) return invalid("mgs_tune_set: unknown dtype");
-  if (!mgs::set_sort_variant(int(w), size_class, mgs::SortVariant{shape, rank_mode})) {
+  if (!mgs::set_sort_variant(int(w), size_class, mgs::SortVariant{shape, rank_mode}, true)) {
     set_last_error("mgs_tune_set: size_class must be in [0, %d), shape in [0, 7), rank_mode 2 or 3",
                    mgs::kSizeClasses);
     return MGS_ERR_INVALID;

@@ -1,7 +1,10 @@
-// Onesweep LSD radix sort for one B200 (sm_100a): the engine's replacement of
-// thrust::sort -> CUB DeviceRadixSort, which the reference calls for every
-// partition / chunk sort (src/tanasic_sort.cuh:264-266,
-// src/gowanlock_sort.cuh:188-190,337-339, src/sort_benchmark.cu:89).
+// Onesweep LSD radix sort for one B200 (sm_100a): the stable sort of the engine,
+// for whatever depends on the input order of equal keys (key-value sorts, bit
+// ranges) and for segments. The plain sort of whole keys, thrust::sort -> CUB
+// DeviceRadixSort in the reference (src/tanasic_sort.cuh:264-266,
+// src/gowanlock_sort.cuh:188-190,337-339, src/sort_benchmark.cu:89), is a
+// partition sort (partition_sort.cu); it runs these kernels where a variant of
+// them is asked for by name (radix_sort, below).
 //
 // Per sort of n keys of w bytes (P = w 8-bit digit passes):
 //   K1 radix_histogram : one streaming read of the keys builds all P digit
@@ -32,6 +35,7 @@
 
 #include "device_common.cuh"
 #include "dispatch.cuh"
+#include "partition_sort.cuh"
 #include "radix_sort.cuh"
 
 namespace mgs {
@@ -1474,7 +1478,9 @@ struct RadixLayout {
 // MGS_ONESWEEP_SHAPE / MGS_RANK_MODE environment variables override the table
 // for experiments.
 constexpr int kDefaultRankMode = 3;
-std::atomic<int> g_variant[2][kSizeClasses];  // shape * 10 + mode; 0 = not set
+std::atomic<int> g_variant[2][kSizeClasses];  // shape * 10 + mode, plus kPinned when asked for; 0 = not set
+constexpr int kPinned = 100;
+std::atomic<uint64_t> g_tile_held{0};  // bit per device: set_wait_control holds a tile back there
 
 int env_override(const char* name, int lo, int hi) {
   const char* e = getenv(name);
@@ -1507,32 +1513,57 @@ void ensure_default_tuning() {
   std::call_once(once, [] { load_default_tuning(); });
 }
 
-bool store_sort_variant(int key_bytes, int size_class_index, SortVariant v) {
+bool store_sort_variant(int key_bytes, int size_class_index, SortVariant v, bool pin) {
   if ((key_bytes != 4 && key_bytes != 8) || size_class_index < 0 || size_class_index >= kSizeClasses ||
       !valid_variant(v))
     return false;
-  g_variant[key_bytes == 8][size_class_index].store(v.shape * 10 + v.mode, std::memory_order_relaxed);
+  g_variant[key_bytes == 8][size_class_index].store(v.shape * 10 + v.mode + (pin ? kPinned : 0),
+                                                      std::memory_order_relaxed);
   return true;
 }
 
-bool set_sort_variant(int key_bytes, int size_class_index, SortVariant v) {
+bool set_sort_variant(int key_bytes, int size_class_index, SortVariant v, bool pin) {
   ensure_default_tuning();  // the default file must not overwrite this entry later
-  return store_sort_variant(key_bytes, size_class_index, v);
+  return store_sort_variant(key_bytes, size_class_index, v, pin);
 }
 
 SortVariant table_variant(int key_bytes, int size_class_index) {
   ensure_default_tuning();
   const int c = size_class_index < 0 ? 0 : (size_class_index >= kSizeClasses ? kSizeClasses - 1 : size_class_index);
-  const int code = g_variant[key_bytes == 8][c].load(std::memory_order_relaxed);
+  const int code = g_variant[key_bytes == 8][c].load(std::memory_order_relaxed) % kPinned;
   return code ? SortVariant{code / 10, code % 10} : SortVariant{kDefaultShape, kDefaultRankMode};
 }
 
+namespace {
+int env_shape() {
+  static const int v = env_override("MGS_ONESWEEP_SHAPE", 0, kNumShapes - 1);
+  return v;
+}
+int env_mode() {
+  static const int v = env_override("MGS_RANK_MODE", 2, 3);
+  return v;
+}
+
+// A plain sort is a partition sort (partition_sort.cu) unless an onesweep
+// variant was asked for by name, through mgs_tune_set or the environment, or a
+// tile is held back: the look-back waits that failure injection lets run out
+// are the onesweep's.
+bool onesweep_wanted(int dtype, size_t n) {
+  const size_t w = dtype_bytes(dtype);
+  if (w == 0 || env_shape() >= 0 || env_mode() >= 0) return true;
+  ensure_default_tuning();
+  if (g_variant[w == 8][size_class(n)].load(std::memory_order_relaxed) >= kPinned) return true;
+  const uint64_t held = g_tile_held.load(std::memory_order_acquire);
+  if (held == 0) return false;
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && ((held >> dev) & 1u);
+}
+}  // namespace
+
 SortVariant sort_variant(int key_bytes, size_t n) {
-  static const int env_shape = env_override("MGS_ONESWEEP_SHAPE", 0, kNumShapes - 1);
-  static const int env_mode = env_override("MGS_RANK_MODE", 2, 3);
   SortVariant v = table_variant(key_bytes, size_class(n));
-  if (env_shape >= 0) v.shape = env_shape;
-  if (env_mode >= 0) v.mode = env_mode;
+  if (env_shape() >= 0) v.shape = env_shape();
+  if (env_mode() >= 0) v.mode = env_mode();
   return v;
 }
 
@@ -1899,13 +1930,24 @@ cudaError_t kway_radix_tiles(int dtype, const void* d_runs, int k, const uint64_
 cudaError_t set_wait_control(uint32_t lookback_spins, uint32_t tma_polls, uint32_t hold_tile) {
   const WaitControl wc{lookback_spins ? lookback_spins : kLookbackSpinLimit, tma_polls ? tma_polls : kTmaWaitLimit,
                        hold_tile, 0u};
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 64) {
+    const uint64_t bit = uint64_t(1) << dev;
+    if (hold_tile != kNoHeldTile) {
+      g_tile_held.fetch_or(bit, std::memory_order_acq_rel);
+    } else {
+      g_tile_held.fetch_and(~bit, std::memory_order_acq_rel);
+    }
+  }
   return cudaMemcpyToSymbol(g_wait_control, &wc, sizeof(wc));
 }
 
 size_t radix_sort_temp_bytes(int dtype, size_t n) {
   size_t bytes = 0;
   dispatch_dtype(dtype, [&](auto tr) { bytes = radix_layout<decltype(tr)>(n).total; });
-  return bytes;
+  return std::max(bytes, partition_sort_temp_bytes(dtype, n));  // either path may run (radix_sort)
 }
 
 size_t radix_sort_pairs_temp_bytes(int dtype, size_t value_bytes, size_t n) {
@@ -2010,6 +2052,7 @@ cudaError_t segmented_sort(int dtype, void* d_keys, size_t n, const uint64_t* d_
 
 cudaError_t radix_sort(int dtype, void* d_keys, size_t n, void* d_temp, size_t temp_bytes, cudaStream_t stream,
                        uint32_t* d_status, LaunchRecorder* rec) {
+  if (!onesweep_wanted(dtype, n)) return partition_sort(dtype, d_keys, n, d_temp, temp_bytes, stream, d_status, rec);
   cudaError_t result = cudaErrorInvalidValue;
   dispatch_dtype(dtype, [&](auto tr) {
     using Tr = decltype(tr);

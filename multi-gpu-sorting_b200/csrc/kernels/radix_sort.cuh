@@ -91,7 +91,9 @@ struct SortVariant {
 int size_class(size_t n);
 size_t size_class_sample(int size_class);  // the key count the autotuner times for a class
 bool valid_variant(SortVariant v);
-bool set_sort_variant(int key_bytes, int size_class, SortVariant v);  // false when out of range
+// false when out of range. pin: plain sorts of that class run this variant from then on (mgs_tune_set); without
+// it the entry is only what the table says, and plain sorts stay partition sorts (partition_sort.cuh).
+bool set_sort_variant(int key_bytes, int size_class, SortVariant v, bool pin);
 SortVariant sort_variant(int key_bytes, size_t n);  // the table's entry, then the environment overrides
 SortVariant table_variant(int key_bytes, int size_class);  // the table's entry alone
 // Tuning files (format in tune.cu): load returns the number of entries read,
@@ -105,7 +107,7 @@ bool save_tuning_file(const char* path);
 // store_sort_variant writes an entry without that step (file reading uses it).
 void ensure_default_tuning();
 void load_default_tuning();
-bool store_sort_variant(int key_bytes, int size_class, SortVariant v);
+bool store_sort_variant(int key_bytes, int size_class, SortVariant v, bool pin);
 
 // Autotuner: for each size class whose sample size is at most max_n, times every
 // variant (CUDA events, median of `reps` sorts of uniformly random keys of the

@@ -82,12 +82,17 @@ cudaError_t autotune(int dtype, size_t max_n, int reps, std::vector<TuneSample>*
     const size_t n = size_class_sample(c);
     if (n > max_n) continue;
     SortVariant best{-1, -1};
+    // Measured variants are pinned so that radix_sort runs them; whatever ends this class leaves none pinned.
+    struct Unpin {
+      int w, c;
+      ~Unpin() { set_sort_variant(w, c, table_variant(w, c), false); }
+    } unpin{int(w), c};
     double best_ms = 1e30;
     const size_t first = out ? out->size() : 0;
     for (int mode = 2; mode <= 3; ++mode) {
       for (int shape = 0; shape < 7; ++shape) {
         const SortVariant v{shape, mode};
-        if (!set_sort_variant(int(w), c, v)) continue;
+        if (!set_sort_variant(int(w), c, v, true)) continue;
         std::vector<float> t;
         for (int r = 0; r <= reps; ++r) {
           e = cudaMemcpyAsync(b.keys, b.pristine, n * w, cudaMemcpyDeviceToDevice, b.stream);
@@ -109,7 +114,7 @@ cudaError_t autotune(int dtype, size_t max_n, int reps, std::vector<TuneSample>*
         }
       }
     }
-    set_sort_variant(int(w), c, best);
+    set_sort_variant(int(w), c, best, false);
     if (out)
       for (size_t i = first; i < out->size(); ++i)
         (*out)[i].chosen = ((*out)[i].variant.shape == best.shape && (*out)[i].variant.mode == best.mode);
@@ -130,7 +135,7 @@ int read_tuning_file(const char* path) {
     char extra;
     const int got = std::sscanf(line, "%d %d %d %d %c", &kb, &c, &shape, &mode, &extra);
     if (got <= 0) continue;  // blank or comment line
-    if (got == 4 && store_sort_variant(kb, c, SortVariant{shape, mode})) {
+    if (got == 4 && store_sort_variant(kb, c, SortVariant{shape, mode}, false)) {
       ++entries;
     } else {
       ++bad;

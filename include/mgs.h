@@ -171,8 +171,8 @@ int mgs_kway_merge_device(mgs_ctx* ctx, int dtype, const void* const* d_runs, co
  * segment inside [0, n). Segments of up to 1024 4-byte / 512 8-byte keys are
  * sorted by one warp, up to one tile (16384 / 8192 keys) by one CTA entirely in
  * shared memory, both classes in one persistent launch; longer segments go
- * through the onesweep passes all at once. The launch sequence does not read
- * anything back to the host (stream-ordered, capturable in a CUDA graph).
+ * through the partition sort (integer keys) or the onesweep passes (IEEE keys)
+ * all at once. The launch sequence does not read anything back to the host (stream-ordered, capturable in a CUDA graph).
  * Invalid offsets (decreasing, or beyond n) leave that segment unsorted and
  * make the next mgs_ctx_synchronize return MGS_ERR_INVALID. Asynchronous. */
 int mgs_segmented_sort_temp_bytes(int dtype, size_t n, size_t num_segments, size_t* bytes);

@@ -500,7 +500,7 @@ __device__ __forceinline__ u32 interval_scale(const Map<B>& m) {
   return xr >= kCoarse ? u32((u64(kCoarse) << 32) / (u64(xr) + 1u)) : 0u;
 }
 
-template <typename B, int KIND, bool RAW>
+template <typename B, int KIND>
 __device__ Map<B> build_map(const B* __restrict__ src, u32 len, MapSmem<B>& sm, u32* scratch) {
   constexpr u32 kPer = kSamples / kThreads;
   const u32 tid = threadIdx.x;
@@ -519,7 +519,7 @@ __device__ Map<B> build_map(const B* __restrict__ src, u32 len, MapSmem<B>& sm, 
 #pragma unroll
   for (u32 i = 0; i < kPer; ++i) {
     if (i < per) {
-      if (RAW) x[i] = one_zero<B, KIND>(to_ordered<B, KIND>(x[i]));
+      x[i] = one_zero<B, KIND>(to_ordered<B, KIND>(x[i]));
       lo = x[i] < lo ? x[i] : lo;
       hi = x[i] > hi ? x[i] : hi;
     }
@@ -737,14 +737,13 @@ __device__ __noinline__ ZeroCounts count_range(const B* __restrict__ p, u32 n, c
   const Map<B> m = sm.map;
   ZeroCounts z{0, 0, 0};
   auto see = [&](B key) {
-    if (ROOT) key = to_ordered<B, KIND>(key);
+    key = to_ordered<B, KIND>(key);
     if (ROOT && KIND == kFloatKey) {
       z.zeros += (key - kNegZero<B>) < B(2) ? 1u : 0u;
       z.neg += key == kNegZero<B> ? 1u : 0u;
       z.below += key < kNegZero<B> ? 1u : 0u;
     }
-    if (ROOT) key = one_zero<B, KIND>(key);
-    return key;
+    return one_zero<B, KIND>(key);
   };
   auto count = [&](u32 cell) { atomicAdd(reinterpret_cast<u32*>(cnt_bytes + cell * step), 1u); };
   const u32 head = min(n, u32((16u - (u32(reinterpret_cast<uintptr_t>(p)) & 15u)) & 15u) / u32(sizeof(B)));
@@ -880,10 +879,10 @@ struct PlanSmem {
 
 // From a segment's cell counts: the cells' first positions (cursor), the units
 // and the next list's segments. to: the list that takes cells that are still
-// too large; root: the segment is the whole caller's array, not yet moved;
+// too large; raw: the segment is the caller's, not yet moved;
 // last: the tail comes next and probes those cells for a second value.
 template <typename B>
-__device__ void plan_segment(const Sort<B>& a, Segment* seg, const Map<B>& m, const MapTable<B>& tab, u32 to, bool root,
+__device__ void plan_segment(const Sort<B>& a, Segment* seg, const Map<B>& m, const MapTable<B>& tab, u32 to, bool raw,
                              bool last, const u32* counts, PlanSmem& sm) {
   constexpr u32 cap = kCap<B>, half = cap / 2;
   const u32 tid = threadIdx.x;
@@ -934,7 +933,7 @@ __device__ void plan_segment(const Sort<B>& a, Segment* seg, const Map<B>& m, co
   __syncthreads();
   const bool identity = sm.identity != 0;  // every key in one cell: it holds one value (lo and hi differ otherwise)
   if (tid == 0) seg->identity = identity ? 1u : 0u;
-  if (identity && root) {  // one value: the caller's array is sorted as it is
+  if (identity && raw) {  // one value: the caller's keys are sorted as they are
     if (tid == 0) a.st->in_place = 1u;
     return;
   }
@@ -1019,7 +1018,7 @@ __global__ __launch_bounds__(kThreads) void part_start_kernel(Sort<B> a, uint4* 
       o->src = 0;
       o->done = 0;
     }
-    const Map<B> m = build_map<B, KIND, true>(a.keys, a.n, sm, scratch);
+    const Map<B> m = build_map<B, KIND>(a.keys, a.n, sm, scratch);
     store_map<B>(a, 0u, m, sm);
     return;
   }
@@ -1046,44 +1045,94 @@ __global__ __launch_bounds__(kThreads, 2) void part_histogram_root_kernel(Sort<B
 }
 
 // The maps of the segments s0, s0 + step, ... of a list.
-template <typename B>
+template <typename B, int KIND>
 __device__ void map_segments(const Sort<B>& a, const Segment* segs, u32 s0, u32 step, u32 nseg, MapSmem<B>& sm,
                              u32* scratch) {
   for (u32 s = s0; s < nseg; s += step) {
     const uint4 q = __ldcg(reinterpret_cast<const uint4*>(segs + s));
     if (__ldcg(&segs[s].done)) continue;
     const B* src = a.buf(__ldcg(&segs[s].src)) + q.x;
-    const Map<B> m = build_map<B, kUnsignedKey, false>(src, q.y, sm, scratch);
+    const Map<B> m = build_map<B, KIND>(src, q.y, sm, scratch);
     store_map<B>(a, s, m, sm);
   }
 }
 
-template <typename B>
+template <typename B, int KIND>
 __global__ __launch_bounds__(kThreads) void part_map_kernel(Sort<B> a) {
   __shared__ MapSmem<B> sm;
   __shared__ __align__(16) u32 scratch[kHistWords];
-  map_segments<B>(a, a.segs(1), blockIdx.x, gridDim.x, u32(__ldcg(&a.st->list[1]) >> 32), sm, scratch);
+  map_segments<B, KIND>(a, a.segs(1), blockIdx.x, gridDim.x, u32(__ldcg(&a.st->list[1]) >> 32), sm, scratch);
+}
+
+// Segmented sort: its large segments as list 1. One block, 1024 segments a
+// round. Segments that do not fit the scratch (they overlap: the offsets are out
+// of order) are left out and reported.
+template <typename B>
+__global__ __launch_bounds__(1024) void part_segments_kernel(Sort<B> a, const u64* __restrict__ offsets,
+                                                             const u32* __restrict__ ids, const u32* __restrict__ count,
+                                                             u32 max_segs, u32 max_tiles) {
+  __shared__ u32 tmp[33];
+  const u32 all = *count, segs = min(all, max_segs);
+  u32 taken = 0, base = 0;
+  bool fits = all <= max_segs;
+  for (u32 r = 0; r < segs; r += 1024u) {
+    const u32 i = r + threadIdx.x;
+    u32 first = 0, len = 0;
+    if (i < segs) {
+      const u32 id = ids[i];
+      first = u32(offsets[id]);
+      len = u32(offsets[id + 1u] - offsets[id]);
+    }
+    const u32 tiles = (len + kTile<B> - 1) / kTile<B>;
+    u32 total;
+    const u32 at = base + block_scan<1024>(tiles, tmp, &total);
+    const bool ok = i < segs && at + tiles <= max_tiles;
+    if (ok) {
+      Segment s;
+      s.start = first;
+      s.len = len;
+      s.tile_base = at;
+      s.cell_base = i * 8u + at * kCellsPerTile<B>;
+      s.src = s.identity = s.done = s.pad = 0u;
+      a.seg1[i] = s;
+    }
+    const u32 n_ok = __syncthreads_count(ok);
+    taken += n_ok;
+    if (n_ok < min(1024u, segs - r)) {  // the first that did not fit ends the list: its tiles are not counted
+      fits = false;
+      break;
+    }
+    base += total;
+  }
+  if (threadIdx.x == 0) {
+    if (taken) {
+      const u32 id = ids[taken - 1u];
+      const u32 tiles = (u32(offsets[id + 1u] - offsets[id]) + kTile<B> - 1) / kTile<B>;
+      a.st->list[1] = (u64(taken) << 32) | (a.seg1[taken - 1u].tile_base + tiles);
+    }
+    if (!fits && a.status != nullptr) atomicOr(a.status, kStatusBadInput);
+  }
 }
 
 // Every segment of list 1.
-template <typename B>
+template <typename B, int KIND>
 __global__ __launch_bounds__(kThreads, 2) void part_histogram_kernel(Sort<B> a) {
   __shared__ HistSmem<B> sm;
   const u64 list = __ldcg(&a.st->list[1]);
   const u32 nseg = u32(list >> 32), tiles = u32(list);
   const u32 t0 = u32(u64(tiles) * blockIdx.x / gridDim.x), t1 = u32(u64(tiles) * (blockIdx.x + 1) / gridDim.x);
-  histogram_tiles<B, kUnsignedKey, false>(a, a.segs(1), nseg, a.count1, t0, t1, sm);
+  histogram_tiles<B, KIND, false>(a, a.segs(1), nseg, a.count1, t0, t1, sm);
 }
 
 template <typename B>
-__global__ __launch_bounds__(kThreads) void part_plan_kernel(Sort<B> a) {
+__global__ __launch_bounds__(kThreads) void part_plan_kernel(Sort<B> a, bool raw) {
   __shared__ PlanSmem sm;
   __shared__ MapTable<B> tab;
   const u32 nseg = u32(__ldcg(&a.st->list[1]) >> 32);
   for (u32 s = blockIdx.x; s < nseg; s += gridDim.x) {
     __syncthreads();
     load_table<B>(tab, a.tables + s);
-    plan_segment<B>(a, a.segs(1) + s, load_map<B>(a.maps + s), tab, 0u, false, true, a.count1, sm);
+    plan_segment<B>(a, a.segs(1) + s, load_map<B>(a.maps + s), tab, 0u, raw, true, a.count1, sm);
   }
 }
 
@@ -1134,7 +1183,7 @@ __device__ __forceinline__ void scatter_tile(const Sort<B>& a, B (&k)[Shape<size
   unsigned char* const key_bytes = reinterpret_cast<unsigned char*>(sm.keys);
   u32 pk[kItems];  // the key's counter (byte offset) | its rank there << 16
   u32 neg_mask = 0;  // the items that are -0.0
-  if (ROOT) {
+  if (KIND != kUnsignedKey) {
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
       k[i] = to_ordered<B, KIND>(k[i]);
@@ -2076,7 +2125,7 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
       a.st->units = 0;
       a.st->list[cur ^ 1u] = 0;
     }
-    map_segments<B>(a, a.segs(cur), b, G, nseg, sm.map.map, sm.map.scratch);
+    map_segments<B, kUnsignedKey>(a, a.segs(cur), b, G, nseg, sm.map.map, sm.map.scratch);
     if (!(ok = grid_barrier(a.st, ++waits * G))) break;
     histogram_tiles<B, kUnsignedKey, false>(a, a.segs(cur), nseg, a.count0, t0, t1, sm.hist);
     if (!(ok = grid_barrier(a.st, ++waits * G))) break;
@@ -2087,7 +2136,7 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
       plan_segment<B>(a, a.segs(cur) + s, load_map<B>(a.maps + s), tab, cur ^ 1u, false, false, a.count0, sm.plan);
     }
     if (!(ok = grid_barrier(a.st, ++waits * G))) break;
-    scatter_tiles<B, KIND, false>(a, a.segs(cur), t0, t1, sm.scatter);
+    scatter_tiles<B, kUnsignedKey, false>(a, a.segs(cur), t0, t1, sm.scatter);
     if (!(ok = grid_barrier(a.st, ++waits * G))) break;
     const u32 units = __ldcg(&a.st->units);
     for (u32 u = b; u < units; u += G) {
@@ -2133,13 +2182,14 @@ struct Layout {
   bool small, two_levels;
 };
 
+// Scratch for n keys; segments > 0: of a segmented sort with that many large segments at most.
 template <typename B, int KIND>
-Layout layout(size_t n) {
+Layout layout(size_t n, size_t segments) {
   Layout L{};
-  L.small = n <= size_t(2 * kThreads) * Shape<sizeof(B)>::kWideItems;
+  L.small = segments == 0 && n <= size_t(2 * kThreads) * Shape<sizeof(B)>::kWideItems;
   if (L.small) return L;
-  L.two_levels = n > kOneLevel<B>;
-  L.max_segs = n / (kWideCap<B> + 1) + 1;
+  L.two_levels = segments > 0 || n > kOneLevel<B>;
+  L.max_segs = std::max(n / (kWideCap<B> + 1) + 1, segments);
   L.max_tiles = n / kTile<B> + L.max_segs + 1;
   const size_t cells = std::max<size_t>(kMaxCells, L.max_segs * 8 + L.max_tiles * kCellsPerTile<B>);
   size_t off = 0;
@@ -2160,12 +2210,36 @@ Layout layout(size_t n) {
   L.maps_off = take(L.max_segs * sizeof(Map<B>));
   L.tables_off = take(L.max_segs * sizeof(MapTable<B>));
   L.tiles_off = take(L.max_tiles * sizeof(uint4));
-  L.units_off = take((8 * (n / (kCap<B> / 2)) + 4096) * sizeof(uint2));
-  L.crowded_off = take((8 * (n / (kCap<B> / 2)) + 4096) * sizeof(uint2));
+  L.units_off = take((8 * (n / (kCap<B> / 2)) + 2 * segments + 4096) * sizeof(uint2));
+  L.crowded_off = take((8 * (n / (kCap<B> / 2)) + 2 * segments + 4096) * sizeof(uint2));
   L.signs_off = KIND == kFloatKey ? take(n / 8 + 8) : 0;
   L.keys_off = take(n * sizeof(B));
   L.total = off;
   return L;
+}
+
+template <typename B>
+Sort<B> make_sort(const Layout& L, B* keys, size_t n, char* tb, uint32_t* d_status) {
+  Sort<B> a;
+  a.keys = keys;
+  a.tmp = reinterpret_cast<B*>(tb + L.keys_off);
+  a.st = reinterpret_cast<State*>(tb);
+  a.seg0 = reinterpret_cast<Segment*>(tb + L.segs_off[0]);
+  a.seg1 = reinterpret_cast<Segment*>(tb + L.segs_off[1]);
+  a.count0 = reinterpret_cast<u32*>(tb + L.counts_off[0]);
+  a.count1 = reinterpret_cast<u32*>(tb + L.counts_off[1]);
+  a.cursor = reinterpret_cast<u32*>(tb + L.cursor_off);
+  a.maps = reinterpret_cast<Map<B>*>(tb + L.maps_off);
+  a.tables = reinterpret_cast<MapTable<B>*>(tb + L.tables_off);
+  a.tiles = reinterpret_cast<uint4*>(tb + L.tiles_off);
+  a.units = reinterpret_cast<uint2*>(tb + L.units_off);
+  a.crowded = reinterpret_cast<uint2*>(tb + L.crowded_off);
+  a.tile_zeros = reinterpret_cast<u32*>(tb + L.zeros_off);
+  a.zero_signs = reinterpret_cast<u32*>(tb + L.signs_off);
+  a.status = d_status;
+  a.n = u32(n);
+  a.last_list = L.two_levels ? 0u : 1u;
+  return a;
 }
 
 struct Device {
@@ -2199,6 +2273,46 @@ cudaError_t launch_scatter(const Sort<B>& a, unsigned grid, cudaStream_t stream,
   return launch_kernel(rec, "part_scatter", kernel, dim3(grid), dim3(kThreads), sizeof(ScatterSmem<B>), stream, a);
 }
 
+// The level of list 1: KIND and raw as in part_histogram_kernel and plan_segment.
+template <typename B, int KIND>
+cudaError_t launch_level(const Sort<B>& a, size_t seg_blocks, bool raw, unsigned sms, cudaStream_t stream,
+                         LaunchRecorder* rec) {
+  cudaError_t e = launch_kernel(rec, "part_map", part_map_kernel<B, KIND>, dim3(unsigned(seg_blocks)), dim3(kThreads), 0,
+                                stream, a);
+  if (e != cudaSuccess) return e;
+  e = launch_kernel(rec, "part_histogram", part_histogram_kernel<B, KIND>, dim3(sms * 2), dim3(kThreads), 0, stream, a);
+  if (e != cudaSuccess) return e;
+  e = launch_kernel(rec, "part_plan", part_plan_kernel<B>, dim3(unsigned(seg_blocks)), dim3(kThreads), 0, stream, a, raw);
+  if (e != cudaSuccess) return e;
+  return launch_scatter<B, KIND, false>(a, sms * Shape<sizeof(B)>::kTileBlocks, stream, rec);
+}
+
+// The units, then whatever is left.
+template <typename B, int KIND>
+cudaError_t launch_units(const Sort<B>& a, size_t max_units, unsigned sms, cudaStream_t stream, LaunchRecorder* rec) {
+  using LShape = Shape<sizeof(B)>;
+  constexpr size_t local_smem = sizeof(LocalSmem<B, LShape::kLocalThreads, LShape::kLocalItems>);
+  auto local = part_local_kernel<B, KIND>;
+  static SmemLimitOnce local_attr;
+  cudaError_t e = local_attr.ensure(local, local_smem);
+  if (e != cudaSuccess) return e;
+  e = launch_kernel(rec, "part_local", local, dim3(unsigned(std::min<size_t>(max_units, size_t(sms) * LShape::kLocalBlocks))),
+                    dim3(LShape::kLocalThreads), local_smem, stream, a);
+  if (e != cudaSuccess) return e;
+  auto tail = part_tail_kernel<B, KIND>;
+  static SmemLimitOnce tail_attr;
+  e = tail_attr.ensure(tail, sizeof(TailSmem<B>));
+  if (e != cudaSuccess) return e;
+  Sort<B> copy = a;
+  u32 cur = a.last_list;
+  void* args[] = {&copy, &cur};
+  if (rec) rec->before("part_tail", stream);
+  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(tail), dim3(sms * 2), dim3(kThreads), args,
+                                  sizeof(TailSmem<B>), stream);
+  if (rec) rec->after("part_tail", stream);
+  return e;
+}
+
 template <typename B, int KIND>
 cudaError_t sort_typed(B* keys, size_t n, void* temp, size_t temp_bytes, cudaStream_t stream, uint32_t* d_status,
                        LaunchRecorder* rec) {
@@ -2206,28 +2320,10 @@ cudaError_t sort_typed(B* keys, size_t n, void* temp, size_t temp_bytes, cudaStr
   constexpr size_t half = size_t(kThreads) * Shape<sizeof(B)>::kWideItems;
   if (n <= half) return launch_small<B, KIND, kThreads>(keys, n, stream, rec);
   if (n <= 2 * half) return launch_small<B, KIND, 2 * kThreads>(keys, n, stream, rec);
-  const Layout L = layout<B, KIND>(n);
+  const Layout L = layout<B, KIND>(n, 0);
   if (temp == nullptr || temp_bytes < L.total) return cudaErrorInvalidValue;
   char* tb = static_cast<char*>(temp);
-  Sort<B> a;
-  a.keys = keys;
-  a.tmp = reinterpret_cast<B*>(tb + L.keys_off);
-  a.st = reinterpret_cast<State*>(tb);
-  a.seg0 = reinterpret_cast<Segment*>(tb + L.segs_off[0]);
-  a.seg1 = reinterpret_cast<Segment*>(tb + L.segs_off[1]);
-  a.count0 = reinterpret_cast<u32*>(tb + L.counts_off[0]);
-  a.count1 = reinterpret_cast<u32*>(tb + L.counts_off[1]);
-  a.cursor = reinterpret_cast<u32*>(tb + L.cursor_off);
-  a.maps = reinterpret_cast<Map<B>*>(tb + L.maps_off);
-  a.tables = reinterpret_cast<MapTable<B>*>(tb + L.tables_off);
-  a.tiles = reinterpret_cast<uint4*>(tb + L.tiles_off);
-  a.units = reinterpret_cast<uint2*>(tb + L.units_off);
-  a.crowded = reinterpret_cast<uint2*>(tb + L.crowded_off);
-  a.tile_zeros = reinterpret_cast<u32*>(tb + L.zeros_off);
-  a.zero_signs = reinterpret_cast<u32*>(tb + L.signs_off);
-  a.status = d_status;
-  a.n = u32(n);
-  a.last_list = L.two_levels ? 0u : 1u;
+  const Sort<B> a = make_sort<B>(L, keys, n, tb, d_status);
   const unsigned sms = unsigned(current_device().sms);
   const size_t tiles = (n + kTile<B> - 1) / kTile<B>;
   const size_t clear_vecs = L.clear_bytes / 16;
@@ -2240,42 +2336,33 @@ cudaError_t sort_typed(B* keys, size_t n, void* temp, size_t temp_bytes, cudaStr
                     stream, a);
   if (e != cudaSuccess) return e;
   e = launch_scatter<B, KIND, true>(a, unsigned(std::min<size_t>(tiles, size_t(sms) * Shape<sizeof(B)>::kTileBlocks)),
-                                 stream, rec);
+                                    stream, rec);
   if (e != cudaSuccess) return e;
   if (L.two_levels) {
-    const size_t segs = std::min<size_t>(L.max_segs, kMaxCells);
-    e = launch_kernel(rec, "part_map", part_map_kernel<B>, dim3(unsigned(segs)), dim3(kThreads), 0, stream, a);
-    if (e != cudaSuccess) return e;
-    e = launch_kernel(rec, "part_histogram", part_histogram_kernel<B>, dim3(sms * 2), dim3(kThreads), 0, stream, a);
-    if (e != cudaSuccess) return e;
-    e = launch_kernel(rec, "part_plan", part_plan_kernel<B>, dim3(unsigned(segs)), dim3(kThreads), 0, stream, a);
-    if (e != cudaSuccess) return e;
-    e = launch_scatter<B, kUnsignedKey, false>(a, sms * Shape<sizeof(B)>::kTileBlocks, stream, rec);
+    e = launch_level<B, kUnsignedKey>(a, std::min<size_t>(L.max_segs, kMaxCells), false, sms, stream, rec);
     if (e != cudaSuccess) return e;
   }
-  using LShape = Shape<sizeof(B)>;
-  constexpr size_t local_smem = sizeof(LocalSmem<B, LShape::kLocalThreads, LShape::kLocalItems>);
-  {
-    auto kernel = part_local_kernel<B, KIND>;
-    static SmemLimitOnce attr;
-    e = attr.ensure(kernel, local_smem);
-    if (e != cudaSuccess) return e;
-    const size_t want = 2 * (n / (kCap<B> / 2)) + 1;
-    e = launch_kernel(rec, "part_local", kernel, dim3(unsigned(std::min<size_t>(want, size_t(sms) * LShape::kLocalBlocks))),
-                      dim3(LShape::kLocalThreads), local_smem, stream, a);
-    if (e != cudaSuccess) return e;
-  }
-  auto kernel = part_tail_kernel<B, KIND>;
-  static SmemLimitOnce attr;
-  e = attr.ensure(kernel, sizeof(TailSmem<B>));
+  return launch_units<B, KIND>(a, 2 * (n / (kCap<B> / 2)) + 1, sms, stream, rec);
+}
+
+// The large segments of a segmented sort: one level apart, what it leaves in the tail.
+template <typename B, int KIND>
+cudaError_t segments_typed(B* keys, size_t n, const u64* offsets, const u32* ids, const u32* count, size_t max_count,
+                           void* temp, size_t temp_bytes, cudaStream_t stream, uint32_t* d_status,
+                           LaunchRecorder* rec) {
+  const Layout L = layout<B, KIND>(n, max_count);
+  if (temp == nullptr || temp_bytes < L.total) return cudaErrorInvalidValue;
+  char* tb = static_cast<char*>(temp);
+  const Sort<B> a = make_sort<B>(L, keys, n, tb, d_status);
+  const unsigned sms = unsigned(current_device().sms);
+  cudaError_t e = cudaMemsetAsync(tb, 0, L.clear_bytes, stream);
   if (e != cudaSuccess) return e;
-  u32 cur = a.last_list;
-  void* args[] = {&a, &cur};
-  if (rec) rec->before("part_tail", stream);
-  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(sms * 2), dim3(kThreads), args,
-                                  sizeof(TailSmem<B>), stream);
-  if (rec) rec->after("part_tail", stream);
-  return e;
+  e = launch_kernel(rec, "part_segments", part_segments_kernel<B>, dim3(1), dim3(1024), 0, stream, a, offsets, ids,
+                    count, u32(max_count), u32(L.max_tiles));
+  if (e != cudaSuccess) return e;
+  e = launch_level<B, KIND>(a, std::min<size_t>(max_count, size_t(sms) * 4), true, sms, stream, rec);
+  if (e != cudaSuccess) return e;
+  return launch_units<B, KIND>(a, 2 * (n / (kCap<B> / 2)) + 1, sms, stream, rec);
 }
 
 }  // namespace
@@ -2284,7 +2371,7 @@ size_t partition_sort_temp_bytes(int dtype, size_t n) {
   size_t bytes = 0;
   dispatch_dtype(dtype, [&](auto tr) {
     using Tr = decltype(tr);
-    bytes = layout<typename Tr::Bits, Tr::kKind>(n).total;
+    bytes = layout<typename Tr::Bits, Tr::kKind>(n, 0).total;
   });
   return bytes;
 }
@@ -2297,6 +2384,29 @@ cudaError_t partition_sort(int dtype, void* d_keys, size_t n, void* d_temp, size
     using Tr = decltype(tr);
     result = sort_typed<typename Tr::Bits, Tr::kKind>(static_cast<typename Tr::Bits*>(d_keys), n, d_temp, temp_bytes,
                                                       stream, d_status, rec);
+  });
+  return result;
+}
+
+size_t partition_segments_temp_bytes(int dtype, size_t n, size_t max_segments) {
+  size_t bytes = 0;
+  dispatch_dtype(dtype, [&](auto tr) {
+    using Tr = decltype(tr);
+    if constexpr (Tr::kKind != kFloatKey) bytes = layout<typename Tr::Bits, Tr::kKind>(n, max_segments).total;
+  });
+  return bytes;
+}
+
+cudaError_t partition_segments(int dtype, void* d_keys, size_t n, const unsigned long long* d_offsets,
+                               const uint32_t* d_ids, const uint32_t* d_count, size_t max_segments, void* d_temp,
+                               size_t temp_bytes, cudaStream_t stream, uint32_t* d_status, LaunchRecorder* rec) {
+  cudaError_t result = cudaErrorInvalidValue;
+  dispatch_dtype(dtype, [&](auto tr) {
+    using Tr = decltype(tr);
+    if constexpr (Tr::kKind != kFloatKey)
+      result = segments_typed<typename Tr::Bits, Tr::kKind>(static_cast<typename Tr::Bits*>(d_keys), n, d_offsets, d_ids,
+                                                            d_count, max_segments, d_temp, temp_bytes, stream, d_status,
+                                                            rec);
   });
   return result;
 }

@@ -58,3 +58,29 @@ def test_partition_sort_matches_oracle(ctx, orc, dtype, kind):
         ctx.sort_device(t.data_ptr(), n, names[dtype])
         ctx.synchronize()
         assert t.cpu().numpy().view(dtype).tobytes() == orc.sort(a).tobytes(), f"{dtype} {kind} n={n}"
+
+
+@pytest.mark.parametrize("dtype", ["u4", "i4", "u8", "i8"])
+def test_large_integer_segments_match_oracle(ctx, orc, dtype):
+    """Segments above one tile of the segmented sort take the partition path for integer keys: every kind of keys,
+    lengths at the path's edges, two levels of cells in one segment, empty and small segments between them."""
+    w = np.dtype(dtype).itemsize
+    tile = {4: 16384, 8: 8192}[w]
+    kinds = ["uniform", "scales", "few", "dense", "clusters", "mostly_one", "zeros"]
+    lens, parts = [], []
+    for i, kind in enumerate(kinds):
+        for n in (tile + 1, 0, 5 * tile + i, 37):
+            lens.append(n)
+            parts.append(keys(dtype, kind, n, np.random.default_rng(100 * i + n)))
+    lens += [ONE_LEVEL[w] + 77, 3 * tile]
+    parts += [keys(dtype, "uniform", lens[-2], np.random.default_rng(1)), np.full(lens[-1], 5, dtype=dtype)]
+    a = np.concatenate(parts)
+    offs = np.zeros(len(lens) + 1, dtype=np.uint64)
+    offs[1:] = np.cumsum(lens)
+    t = torch.from_numpy(a.view(np.int32 if w == 4 else np.int64).copy()).cuda()
+    o = torch.from_numpy(offs.view(np.int64)).cuda()
+    torch.cuda.synchronize()
+    names = {"u4": "u32", "i4": "i32", "u8": "u64", "i8": "i64"}
+    ctx.segmented_sort_device(t.data_ptr(), a.size, o.data_ptr(), len(lens), names[dtype])
+    ctx.synchronize()
+    assert t.cpu().numpy().view(dtype).tobytes() == orc.segmented_sort(a, offs).tobytes()

@@ -12,6 +12,8 @@
 //                        its runs, then ties split by run index (stable).
 //                        Hierarchical: coarser levels (every 256, then every
 //                        16 tiles) bound the finer searches.
+//   kway_unit_tiles    : (partition_sort.cu) per output tile of a k-way merge of
+//                        integer keys, the slices sorted by bins.
 //   K5/K7b tile_merge  : per output tile, the k input ranges are staged in shared
 //                        memory in run order and merged by ceil(log2 k) rounds of
 //                        pairwise merge-path merges in shared memory, then stored
@@ -28,6 +30,7 @@
 #include "device_common.cuh"
 #include "dispatch.cuh"
 #include "merge.cuh"
+#include "partition_sort.cuh"
 #include "radix_sort.cuh"
 
 namespace mgs {
@@ -114,7 +117,8 @@ __device__ __forceinline__ u64 bound_search(const typename Tr::Bits* run, u64 lo
 }
 
 constexpr int kMaxRunsPerLane = kMaxKwayRuns / 32;
-static_assert(kMaxKwayTileRuns >= kMaxKwayRuns, "the radix tiles take every k-way merge");
+static_assert(kMaxKwayTileRuns >= kMaxKwayRuns && kMaxUnitTileRuns >= kMaxKwayRuns,
+              "the sorted tiles take every k-way merge");
 
 // One warp per diagonal d: splits[r] = number of elements of run r among the
 // first d outputs of the stable k-way merge. Optional coarse level: the
@@ -484,12 +488,34 @@ int kway_radix_min_runs() {
   return env >= 0 ? (env == 0 ? kMaxKwayRuns + 1 : env) : 24;
 }
 
-// Output tile of a k-way merge: a radix tile or a merge tile.
+// Merges of at least this many runs of integer keys sort their tiles like the
+// units of the partition sort (kway_unit_tiles): one placing by bins, whatever k
+// is, instead of ceil(log2 k) merge rounds. Measured on a B200, Dirichlet(1)
+// runs, merged or radix tiles against these, partition included: 2^27 uint32,
+// k = 3: 955 / 922 us, 8: 1178 / 956, 16: 1381 / 1004, 64: 2258 / 1479; 2^26
+// int64, k = 16: 1320 / 1292 (nearly sorted keys 1152 / 1252), 32: 1588 / 1387,
+// 64: 2075 / 1707. MGS_KWAY_UNIT_MIN_RUNS overrides it for experiments (0: never).
+int kway_unit_min_runs(size_t key_bytes) {
+  static const int env = [] {
+    const char* e = getenv("MGS_KWAY_UNIT_MIN_RUNS");
+    return e ? atoi(e) : -1;
+  }();
+  if (env >= 0) return env == 0 ? kMaxKwayRuns + 1 : env;
+  return key_bytes == 4 ? 3 : 32;
+}
+
+// Output tile of a k-way merge: how it is made, and its keys.
+enum class KwayTile { kMerge, kRadix, kUnit };
 template <class Tr>
-u64 kway_tile_keys(int k, bool* radix) {
+u64 kway_tile_keys(int k, KwayTile* how) {
+  const size_t ut = kway_unit_tile_keys(dtype_of<Tr>());
   const size_t rt = kway_radix_tile_keys(dtype_of<Tr>());
-  *radix = k > 2 && rt != 0 && k >= kway_radix_min_runs();
-  return *radix ? u64(rt) : merge_tile_keys(sizeof(typename Tr::Bits), merge_shape(k));
+  if (k > 2 && ut != 0 && k >= kway_unit_min_runs(sizeof(typename Tr::Bits))) {
+    *how = KwayTile::kUnit;
+    return u64(ut);
+  }
+  *how = k > 2 && rt != 0 && k >= kway_radix_min_runs() ? KwayTile::kRadix : KwayTile::kMerge;
+  return *how == KwayTile::kRadix ? u64(rt) : merge_tile_keys(sizeof(typename Tr::Bits), merge_shape(k));
 }
 
 // The exact splits of a k-way merge (k > 2) are found level by level: every
@@ -507,13 +533,13 @@ struct KwayLayout {
   size_t b_splits_off[kBoundLevels], b_ub_off[kBoundLevels], b_lt_off[kBoundLevels], b_vstar_off[kBoundLevels];
   u64 tile, num_tiles;
   u64 b_diag[kBoundLevels];  // diagonals of each bounding level (0: level absent)
-  bool radix;
+  KwayTile how;
 };
 
 template <class Tr>
 KwayLayout kway_layout(int k, size_t total) {
   KwayLayout L;
-  const u64 kTile = kway_tile_keys<Tr>(k, &L.radix);
+  const u64 kTile = kway_tile_keys<Tr>(k, &L.how);
   L.tile = kTile;
   L.num_tiles = (total + kTile - 1) / kTile;
   size_t off = 0;
@@ -656,14 +682,15 @@ cudaError_t kway_merge_typed(const void* const* runs_v, const size_t* lens, int 
   if (e != cudaSuccess) return e;
   const Bits* const* cruns = d_runs;
   const u64* csplits = d_splits;
-  if (L.radix) {
+  if (L.how != KwayTile::kMerge) {
     // Output tiles in windows of about window_keys keys (one window when 0), as launch_tile_merges.
     const u64 per_window =
         window_keys == 0 ? L.num_tiles : std::max<u64>(1, (u64(window_keys) + kTile - 1) / kTile);
     for (u64 t0 = 0; t0 < L.num_tiles; t0 += per_window) {
       const u64 t1 = std::min<u64>(L.num_tiles, t0 + per_window);
-      e = kway_radix_tiles(dtype_of<Tr>(), cruns, k, reinterpret_cast<const uint64_t*>(d_splits), out, u64(total), t0,
-                           t1 - t0, stream, rec);
+      auto tiles = L.how == KwayTile::kUnit ? kway_unit_tiles : kway_radix_tiles;
+      e = tiles(dtype_of<Tr>(), cruns, k, reinterpret_cast<const uint64_t*>(d_splits), out, u64(total), t0, t1 - t0,
+                stream, rec);
       if (e != cudaSuccess) return e;
       if (on_window) {
         const u64 first = t0 * kTile, last = std::min<u64>(total, t1 * kTile);

@@ -2034,6 +2034,100 @@ __global__ __launch_bounds__(THREADS, 1) void part_small_kernel(B* keys, u32 n) 
   store_unit<B, KIND, THREADS, ITEMS>(keys, n, sm);
 }
 
+// ---------------------------------------------------------------- merge -----
+// One output tile of a k-way merge of integer keys: the tile's slice of every
+// run (from the split matrix) is read in run order and sorted like a unit; equal
+// keys are the same bytes, so the merge's order among them does not show.
+// Tiles of kWideCap keys: half as many splits to find as with the units' blocks.
+// 2^28 uint32, 16 runs: 1.19 ms against 1.96 ms of four merge rounds.
+template <typename B, int KIND>
+__global__ __launch_bounds__(kThreads, 2) void kway_unit_tile_kernel(const B* const* __restrict__ runs, int k,
+                                                                     const u64* __restrict__ splits,
+                                                                     B* __restrict__ out, u64 total, u64 tile0) {
+  constexpr int ITEMS = Shape<sizeof(B)>::kWideItems;
+  using Smem = LocalSmem<B, kThreads, ITEMS>;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+  const B** sptr = reinterpret_cast<const B**>(smem_raw + (sizeof(Smem) + 15) / 16 * 16);  // slice r's first key - seg0[r]
+  u32* seg0 = reinterpret_cast<u32*>(sptr + k);  // slice offsets in the tile (k + 1)
+  const u32 tid = threadIdx.x;
+  const u64 j = tile0 + blockIdx.x;
+  const u64 d0 = j * u64(kWideCap<B>);
+  const u32 cnt = u32(min(u64(kWideCap<B>), total - d0));
+  const u32 per_thread = (u32(k) + kThreads - 1u) / kThreads;
+  u32 local = 0;
+  for (u32 i = 0; i < per_thread; ++i) {
+    const u32 r = tid * per_thread + i;
+    if (r < u32(k)) local += u32(splits[(j + 1) * k + r] - splits[j * k + r]);
+  }
+  u32 tot;
+  u32 at = block_scan<kThreads>(local, sm.tmp[0], &tot);
+  for (u32 i = 0; i < per_thread; ++i) {
+    const u32 r = tid * per_thread + i;
+    if (r < u32(k)) {
+      const u64 s = splits[j * k + r];
+      seg0[r] = at;
+      sptr[r] = runs[r] + s - at;
+      at += u32(splits[(j + 1) * k + r] - s);
+    }
+  }
+  if (tid == 0) seg0[k] = cnt;
+  __syncthreads();
+  // Consecutive threads read consecutive keys; a thread's slice only moves forward (its keys are kThreads apart).
+  B key[ITEMS];
+  {
+    u32 r = 0, hi = u32(k);  // the largest r with seg0[r] <= tid
+    while (hi - r > 1u) {
+      const u32 mid = (r + hi) >> 1;
+      if (seg0[mid] <= tid) {
+        r = mid;
+      } else {
+        hi = mid;
+      }
+    }
+    u32 end = seg0[r + 1u];
+    const B* base = sptr[r];
+#pragma unroll
+    for (int t = 0; t < ITEMS; ++t) {
+      const u32 i = u32(t) * kThreads + tid;
+      if (i < cnt) {
+        if (i >= end) {
+          do {
+            ++r;
+          } while (seg0[r + 1u] <= i);  // seg0[k] = cnt > i ends the walk
+          end = seg0[r + 1u];
+          base = sptr[r];
+        }
+        key[t] = __ldg(base + i);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < ITEMS; ++t) key[t] = to_ordered<B, KIND>(key[t]);
+  u32 rounds = place_keys<B, kThreads, ITEMS>(key, cnt, sm);
+  if (rounds == kOneValue) {
+    const B one = from_ordered<B, KIND>(key[0]);
+    for (u32 i = tid; i < cnt; i += kThreads) out[d0 + i] = one;
+    return;
+  }
+  finish_order<B, kThreads, ITEMS>(cnt, rounds, sm);
+  if (rounds > kBinLimit<B>) {
+    bool done = in_order<B, kThreads, ITEMS>(cnt, sm);
+    for (u32 tries = 0; !done && tries < 2u; ++tries) {
+      finish_order<B, kThreads, ITEMS>(cnt, rounds, sm);
+      done = in_order<B, kThreads, ITEMS>(cnt, sm);
+    }
+    if (!done) {  // crowded bins: the staged keys go out as they are and come back through the output
+      store_unit<B, KIND, kThreads, ITEMS>(out + d0, cnt, sm);
+      __threadfence_block();
+      __syncthreads();
+      rounds = place_crowded<B, KIND, true, kThreads, ITEMS>(out + d0, cnt, sm);
+      finish_order<B, kThreads, ITEMS>(cnt, rounds, sm);
+    }
+  }
+  store_unit<B, KIND, kThreads, ITEMS>(out + d0, cnt, sm);
+}
+
 // ---------------------------------------------------------------- P4 --------
 template <typename B>
 union TailSmem {
@@ -2407,6 +2501,36 @@ cudaError_t partition_segments(int dtype, void* d_keys, size_t n, const unsigned
       result = segments_typed<typename Tr::Bits, Tr::kKind>(static_cast<typename Tr::Bits*>(d_keys), n, d_offsets, d_ids,
                                                             d_count, max_segments, d_temp, temp_bytes, stream, d_status,
                                                             rec);
+  });
+  return result;
+}
+
+size_t kway_unit_tile_keys(int dtype) {
+  size_t keys = 0;
+  dispatch_dtype(dtype, [&](auto tr) {
+    using Tr = decltype(tr);
+    if constexpr (Tr::kKind != kFloatKey) keys = kWideCap<typename Tr::Bits>;
+  });
+  return keys;
+}
+
+cudaError_t kway_unit_tiles(int dtype, const void* d_runs, int k, const uint64_t* d_splits, void* out, uint64_t total,
+                            uint64_t tile0, uint64_t tiles, cudaStream_t stream, LaunchRecorder* rec) {
+  cudaError_t result = cudaErrorInvalidValue;
+  if (k < 1 || k > kMaxUnitTileRuns || tiles == 0 || tiles > 0x7FFFFFFFull) return result;
+  dispatch_dtype(dtype, [&](auto tr) {
+    using Tr = decltype(tr);
+    using B = typename Tr::Bits;
+    if constexpr (Tr::kKind != kFloatKey) {
+      auto kernel = kway_unit_tile_kernel<B, Tr::kKind>;
+      constexpr size_t base = (sizeof(LocalSmem<B, kThreads, Shape<sizeof(B)>::kWideItems>) + 15) / 16 * 16;
+      static SmemLimitOnce attr;
+      result = attr.ensure(kernel, base + size_t(kMaxUnitTileRuns) * 12 + 4);
+      if (result != cudaSuccess) return;
+      result = launch_kernel(rec, "kway_unit_tiles", kernel, dim3(unsigned(tiles)), dim3(kThreads),
+                             base + size_t(k) * 12 + 4, stream, static_cast<const B* const*>(d_runs), k,
+                             reinterpret_cast<const u64*>(d_splits), static_cast<B*>(out), u64(total), u64(tile0));
+    }
   });
   return result;
 }

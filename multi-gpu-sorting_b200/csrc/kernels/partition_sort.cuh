@@ -29,4 +29,14 @@ cudaError_t partition_segments(int dtype, void* d_keys, size_t n, const unsigned
                                const uint32_t* d_ids, const uint32_t* d_count, size_t max_segments, void* d_temp,
                                size_t temp_bytes, cudaStream_t stream, uint32_t* d_status, LaunchRecorder* rec);
 
+// K-way merge tiles of integer keys, sorted in shared memory: tile j in [tile0,
+// tile0 + tiles) of the output is out[j*T, (j+1)*T) (T = kway_unit_tile_keys,
+// the last tile shorter; 0 for IEEE types), from the slices splits[j*k + r] ..
+// splits[(j+1)*k + r) of the k device runs (d_runs: a device array of k run
+// pointers; splits: a (tiles + 1) x k device matrix at spacing T).
+constexpr int kMaxUnitTileRuns = 1024;
+size_t kway_unit_tile_keys(int dtype);
+cudaError_t kway_unit_tiles(int dtype, const void* d_runs, int k, const uint64_t* d_splits, void* out, uint64_t total,
+                            uint64_t tile0, uint64_t tiles, cudaStream_t stream, LaunchRecorder* rec);
+
 }  // namespace mgs

@@ -15,6 +15,8 @@ ONE_LEVEL = {4: 1022 * 3584, 8: 1022 * 2506}  # keys that one level of cells tak
 
 def keys(dtype, kind, n, rng):
     dt = np.dtype(dtype)
+    if n == 0:
+        return np.empty(0, dt)
     bits = 8 * dt.itemsize
     u = np.dtype(f"u{dt.itemsize}")
     full = rng.integers(0, 1 << bits, n, dtype=u, endpoint=False) if bits < 64 else \

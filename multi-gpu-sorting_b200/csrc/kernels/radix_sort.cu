@@ -1878,37 +1878,38 @@ cudaError_t segmented_sort_typed(typename Tr::Bits* keys, size_t n, const uint64
   if constexpr (kSegmentsPartitioned(Tr::kKind)) {
     return partition_segments((sizeof(Bits) == 4 ? 0 : 3) + Tr::kKind, keys, n, offs, large_ids, hdr->counts + 2,
                               L.max_large, tb + L.keys_off, L.total - L.keys_off, stream, d_status, rec);
-  }
-  SegLarge sg{offs, large_ids, prefix, hdr->counts, bucket, tile_info};
-  {
-    auto kernel = seg_histogram_kernel<Tr, PlainDigits>;
-    static SmemLimitOnce attr;
-    e = attr.ensure(kernel, HistCopies<Tr>::kSmemBytes);
-    if (e != cudaSuccess) return e;
-    e = launch_kernel(rec, "seg_histogram", kernel, dim3(unsigned(sms)), dim3(kHistBlock), HistCopies<Tr>::kSmemBytes,
-                      stream, static_cast<const Bits*>(keys), sg, kTile, hist, lb[0], tile_info, PlainDigits{});
-    if (e != cudaSuccess) return e;
-  }
-  e = launch_kernel(rec, "seg_scan", seg_scan_kernel<Tr::kPasses>, dim3(unsigned(sms * 4)), dim3(kRadix), 0, stream,
-                    static_cast<const uint32_t*>(hdr->counts), static_cast<const uint32_t*>(hist), bucket);
-  if (e != cudaSuccess) return e;
-  {
-    auto kernel = radix_onesweep_kernel<Tr, Shape::kBlock, Shape::kItems, Shape::kMinBlocks, Shape::kChains,
-                                        uint32_t, 3, true>;
-    static SmemLimitOnce attr;
-    e = attr.ensure(kernel, sizeof(Smem));
-    if (e != cudaSuccess) return e;
-    for (int p = 0; p < Tr::kPasses; ++p) {
-      uint32_t* next = (p + 1 < Tr::kPasses) ? lb[(p + 1) & 1] : nullptr;
-      e = launch_kernel(rec, "seg_onesweep", kernel, dim3(unsigned(sms)), dim3(Shape::kBlock), sizeof(Smem), stream,
-                        keys, tmp, st, lb[p & 1], next, uint32_t(n), 0u, p, 1, sg, static_cast<NoValue*>(nullptr),
-                        static_cast<NoValue*>(nullptr), PlainDigits{});
+  } else {
+    SegLarge sg{offs, large_ids, prefix, hdr->counts, bucket, tile_info};
+    {
+      auto kernel = seg_histogram_kernel<Tr, PlainDigits>;
+      static SmemLimitOnce attr;
+      e = attr.ensure(kernel, HistCopies<Tr>::kSmemBytes);
+      if (e != cudaSuccess) return e;
+      e = launch_kernel(rec, "seg_histogram", kernel, dim3(unsigned(sms)), dim3(kHistBlock), HistCopies<Tr>::kSmemBytes,
+                        stream, static_cast<const Bits*>(keys), sg, kTile, hist, lb[0], tile_info, PlainDigits{});
       if (e != cudaSuccess) return e;
     }
+    e = launch_kernel(rec, "seg_scan", seg_scan_kernel<Tr::kPasses>, dim3(unsigned(sms * 4)), dim3(kRadix), 0, stream,
+                      static_cast<const uint32_t*>(hdr->counts), static_cast<const uint32_t*>(hist), bucket);
+    if (e != cudaSuccess) return e;
+    {
+      auto kernel = radix_onesweep_kernel<Tr, Shape::kBlock, Shape::kItems, Shape::kMinBlocks, Shape::kChains,
+                                          uint32_t, 3, true>;
+      static SmemLimitOnce attr;
+      e = attr.ensure(kernel, sizeof(Smem));
+      if (e != cudaSuccess) return e;
+      for (int p = 0; p < Tr::kPasses; ++p) {
+        uint32_t* next = (p + 1 < Tr::kPasses) ? lb[(p + 1) & 1] : nullptr;
+        e = launch_kernel(rec, "seg_onesweep", kernel, dim3(unsigned(sms)), dim3(Shape::kBlock), sizeof(Smem), stream,
+                          keys, tmp, st, lb[p & 1], next, uint32_t(n), 0u, p, 1, sg, static_cast<NoValue*>(nullptr),
+                          static_cast<NoValue*>(nullptr), PlainDigits{});
+        if (e != cudaSuccess) return e;
+      }
+    }
+    // Passes are never skipped here (an even number ran): only the status report.
+    return launch_kernel(rec, "radix_finalize", radix_finalize_kernel<Tr>, dim3(1), dim3(256), 0, stream, keys,
+                         static_cast<const Bits*>(tmp), static_cast<const RadixState*>(st), 0u, d_status);
   }
-  // Passes are never skipped here (an even number ran): only the status report.
-  return launch_kernel(rec, "radix_finalize", radix_finalize_kernel<Tr>, dim3(1), dim3(256), 0, stream, keys,
-                       static_cast<const Bits*>(tmp), static_cast<const RadixState*>(st), 0u, d_status);
 }
 
 }  // namespace

@@ -30,9 +30,9 @@
 // on a B200 (B200 copy peak 6.45 TB/s), against the 8-bit passes: 2^30 uniform
 // uint32 15.5 -> 12.1 ms, 10^8 normal float64 4.7 -> 2.4 ms, 2^20 int64 below
 // 10^6 83 -> 50 us, 50021 normal float32 60 -> 50 us, 1000 uint32 50 -> 13 us.
-// part_histogram reads at 6.4 TB/s. part_scatter (24 SM cycles per 32 keys) and
-// part_local (31) are bound by the shared-memory pipe and its latency: a scatter
-// issues 12.5 shared wavefronts and 38 instructions per 32 keys, where the
+// part_histogram reads at 6.4 TB/s. part_scatter (22 SM cycles per 32 keys) and
+// part_local (32) are bound by the shared-memory pipe and its latency: a scatter
+// issues 14 shared wavefronts and 37-40 instructions per 32 keys, where the
 // stable ranking of the 8-bit passes issues 24 and 63.
 //
 // IEEE zeros: -0.0 and +0.0 are equal keys with different bytes and keep their
@@ -71,9 +71,15 @@ constexpr u32 kBarrierSpins = 1u << 25;
 // with 512 x 20 keys and two blocks per SM 1.39 ms, 256 x 28 and three 1.37 ms,
 // 384 x 20 and three 1.39 ms, 256 x 20 and four 1.27 ms (same code, before the
 // call on crowded bins was moved out of it).
-// kTileItems keys per thread make a scatter tile, kTileBlocks blocks per SM;
-// more items, or three blocks of fewer, spill: 2^28 uint32, both scatters with
-// 16 items and two blocks 1.40 ms, 24 and two 1.78 ms, 12 and three 1.83 ms.
+// kTileItems keys per thread make a scatter tile, kTileBlocks blocks per SM: a
+// larger tile has longer runs per cell and fewer global atomics per key, until
+// its keys spill. 2^28 uint32, both scatters: 16 items and two blocks 1.43 ms,
+// 18 and two 1.43, 20 and two 1.64, 24 and two 2.08, 12 and three 1.83. 8-byte
+// keys, whole sorts of 2^20 int64 / 10^8 float64 / 2^28 uint64: 8 items 54 us /
+// 2.63 / 5.11 ms, 10 items 56 us / 2.62 / 5.00 ms.
+// 256 x 20 keys and four blocks against 512 x 20 and two in part_local, whole
+// sorts: 2^24 uint32 237 / 239 us, 2^26 float32 0.945 / 1.03 ms, 2^28 uint32
+// 2.85 / 2.88 ms, 2^30 uint32 12.15 / 11.74 ms: only the largest would gain.
 template <int W>
 struct Shape;
 template <>

@@ -1357,11 +1357,13 @@ constexpr u32 kBinLimit = sizeof(B) == 4 ? 8 : 7;
 template <typename B>
 constexpr u32 kBorder = sizeof(B) == 4 ? 8 : 6;
 constexpr u32 kWarpPart = 256;  // crowded parts up to this size are sorted by a warp
+constexpr u32 kExactBits = 15;  // Bins gives every value a bin of its own for ranges below 2^kExactBits
 
 template <typename B, int THREADS, int ITEMS>
 struct LocalSmem {
   static constexpr u32 kKeys = u32(THREADS) * ITEMS;
   static constexpr u32 kBins = u32(ITEMS + 3) / 4u * 4u * THREADS;  // a bin per key
+  static_assert(kBins <= 1u << kExactBits, "a range below the bins' number must fit the exact bins");
   static constexpr u32 kParts = kKeys / (kBinLimit<B> + 1) + 1, kBigParts = kKeys / (kWarpPart + 1) + 1;
   alignas(16) B keys[kKeys + 16];
   alignas(16) u32 bins[kBins + 4];
@@ -1541,9 +1543,10 @@ struct Bins {
       shift = lz < 32 ? u32(32 - lz) : 0u;
     }
     exact = range < B(nbins);
-    mul = exact ? 1u << 18 : 1u;  // d * 2^18 * 2^14 / 2^32 = d
+    // Exact: d * 2^17 * 2^15 / 2^32 = d. Both products must fit: d < nbins <= 2^15 (checked in LocalSmem).
+    mul = exact ? 1u << (32 - kExactBits) : 1u;
     const u32 most = MAY_LOG && log ? log_x(range) : u32(range >> shift);
-    scale = exact ? 1u << 14 : u32(float(nbins) * (4294967296.f * 0.9999995f) / (float(most) + 1.f));
+    scale = exact ? 1u << kExactBits : u32(float(nbins) * (4294967296.f * 0.9999995f) / (float(most) + 1.f));
   }
   // bin in the high word, position within the bin (a 32-bit fraction) in the low word
   __device__ __forceinline__ u64 product(B key) const {

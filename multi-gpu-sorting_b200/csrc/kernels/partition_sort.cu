@@ -283,11 +283,22 @@ __device__ u32 any_cell_of(const Map<B>& m, const MapTable<B>& tab, B key) {
   return c;
 }
 
-// One value for every key of a cell?
+// One value for every key of a cell? True only where the map proves it for every
+// key, sampled or not: such a cell's keys are copied as they are, and nothing
+// looks at them again.
+//   kSplit : keys of a cell between two edges lie in [edge, next edge).
+//   kTable : offsets and logarithms send every key outside the sampled range to
+//            the first or the last cell, and so do 4-byte keys themselves: the
+//            other cells are made of offsets in [0, range], searched below.
+//            High words (8-byte kPlain) bound neither end of the sample, and a
+//            cell that takes a high word takes all 2^32 keys that have it.
+//   kLinear: the end cells take what lies outside, and every cell spans four
+//            values or more (a linear map needs 4 * kMaxCells of them).
 template <typename B>
 __device__ __noinline__ bool cell_is_one_value(const Map<B>& m, const MapTable<B>& tab, u32 cell) {
   if (cell == 0u || cell == m.ncells - 1u) return false;  // may hold keys outside the sampled range
   if (m.kind == kSplit) return tab.edge[cell] - tab.edge[cell - 1u] == 1;
+  if (m.kind == kLinear || (sizeof(B) == 8 && m.xmode == kPlain)) return false;
   auto cell_at = [&](B d) { return any_cell_of<B>(m, tab, m.lo + d); };
   B first[2];
   for (u32 q = 0; q < 2; ++q) {  // the smallest offset with a cell >= cell + q
@@ -937,7 +948,11 @@ __device__ void plan_segment(const Sort<B>& a, Segment* seg, const Map<B>& m, co
   }
   if (tid == 0) sm.start[runs] = len;
   __syncthreads();
-  const bool identity = sm.identity != 0;  // every key in one cell: it holds one value (lo and hi differ otherwise)
+  // Every key in one cell: it holds one value. Were there two, the smallest and the largest sampled key would differ
+  // and have different cells (a table gives x_lo cell 1 and x_hi cell ncells - 2; equal cells over more than 4096
+  // values part them; the second edge of a split lies above the first and not above its largest sample); and if all
+  // samples are one value, every map of a range of one value sends the keys below and above it to other cells.
+  const bool identity = sm.identity != 0;
   if (tid == 0) seg->identity = identity ? 1u : 0u;
   if (identity && raw) {  // one value: the caller's keys are sorted as they are
     if (tid == 0) a.st->in_place = 1u;

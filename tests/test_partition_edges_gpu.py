@@ -30,3 +30,48 @@ def test_dense_keys_match_oracle(ctx, orc, dtype):
             ids = np.arange(n) if top == n - 1 else np.append(rng.integers(0, top + 1, n - 2), [0, top])
             a = rng.permutation(ids + offset).astype(u).view(dtype)
             assert sorted_on_device(ctx, a).tobytes() == orc.sort(a).tobytes(), f"{dtype} n={n} range={top}"
+
+
+def heavy_end(kind, n, rng):
+    """8-byte keys half of which are the largest (or, mirrored, the smallest) value that a sample of them shows, with a
+    few others beyond it that agree with it in their high word and that a sample most likely misses."""
+    if kind == "clipped":  # cosine similarities clipped to 1.0, and a few just above it
+        a = rng.uniform(0.94, 1.0, n)
+        a[rng.permutation(n)[:n // 2]] = 1.0
+        a[rng.permutation(n)[:5]] = 1.0 + 2.0 ** -52
+    else:  # ids in the high word; low words of their own for a few keys of the most frequent id
+        a = rng.integers(0, 100_000, n, dtype=np.uint64) << np.uint64(32)
+        heavy = np.uint64(100_000 << 32)
+        a[rng.permutation(n)[:n // 2]] = heavy
+        a[rng.permutation(n)[:3]] = heavy + np.array([9, 5, 7], dtype=np.uint64)
+    return a
+
+
+def mirrored(a):
+    return -a if a.dtype.kind == "f" else ~a
+
+
+@pytest.mark.parametrize("n", [1 << 20, 2_000_000, 10_000_000])
+@pytest.mark.parametrize("kind,dtype", [("clipped", "f8"), ("ids", "u8"), ("ids", "i8"), ("ids", "f8")])
+def test_heavy_end_values_match_oracle(ctx, orc, kind, dtype, n):
+    a = heavy_end(kind, n, np.random.default_rng(n))
+    for b in (a, mirrored(a)):
+        b = b.view(dtype)
+        assert sorted_on_device(ctx, b).tobytes() == orc.sort(b).tobytes()
+
+
+@pytest.mark.parametrize("dtype", ["u8", "i8"])
+def test_heavy_end_values_in_large_segments_match_oracle(ctx, orc, dtype):
+    rng = np.random.default_rng(5)
+    parts = []
+    for n in (20_000, 1 << 20, 300_001, 3_000_000):
+        a = heavy_end("ids", n, rng)
+        parts += [a.view(dtype), mirrored(a).view(dtype)]
+    a = np.concatenate(parts)
+    offs = np.concatenate([[0], np.cumsum([p.size for p in parts])]).astype(np.uint64)
+    t = torch.from_numpy(a.view(np.int64).copy()).cuda()
+    o = torch.from_numpy(offs.view(np.int64)).cuda()
+    torch.cuda.synchronize()
+    ctx.segmented_sort_device(t.data_ptr(), a.size, o.data_ptr(), len(parts), NAMES[dtype])
+    ctx.synchronize()
+    assert t.cpu().numpy().view(dtype).tobytes() == orc.segmented_sort(a, offs).tobytes()

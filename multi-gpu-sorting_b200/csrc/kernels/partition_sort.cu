@@ -96,6 +96,10 @@ struct Shape<8> {
 };
 template <typename B>
 constexpr u32 kTile = u32(kThreads) * Shape<sizeof(B)>::kTileItems;
+// Parts of `per` keys in len keys, the last one shorter. (len + per - 1) / per
+// would wrap for the largest sorts: len may be any number below 2^32.
+__host__ __device__ constexpr u32 parts_of(u32 len, u32 per) { return len / per + (len % per != 0u ? 1u : 0u); }
+static_assert(parts_of(~0u, 8192u) == 524288u && parts_of(~0u, ~0u) == 1u && parts_of(0u, 8u) == 0u, "no wrap");
 template <typename B>
 constexpr u32 kCap = u32(Shape<sizeof(B)>::kLocalThreads) * Shape<sizeof(B)>::kLocalItems;
 template <typename B>
@@ -483,7 +487,7 @@ constexpr u32 kOneLevel = (kMaxCells - 2u) * kCellUniform<B>;
 // split evenly, times `more` (of a table's cells many hold few keys or none).
 template <typename B>
 __device__ __forceinline__ u32 inner_cells(u32 len, u32 per, u32 more) {
-  u32 need = (len + per - 1) / per;
+  u32 need = parts_of(len, per);
   if (need > kMaxCells - 2u)
     need = len <= kOneLevel<B> ? kMaxCells - 2u : min(kMaxCells - 2u, more * u32(sqrtf(float(need)) + 1.f));
   return max(need, 4u);  // the smallest and the largest sampled key get different cells
@@ -827,7 +831,7 @@ __device__ void histogram_tiles(const Sort<B>& a, const Segment* segs, u32 nseg,
     const uint4 head = ROOT ? make_uint4(0u, a.n, 0u, 0u) : __ldcg(reinterpret_cast<const uint4*>(segs + s));
     const u32 start = head.x, len = head.y, tile_base = head.z, cell_base = head.w;
     const u32 buf = ROOT ? 0u : __ldcg(&segs[s].src);
-    const u32 e = min(t1, tile_base + (len + kTile<B> - 1) / kTile<B>);
+    const u32 e = min(t1, tile_base + parts_of(len, kTile<B>));
     if (!ROOT) {
       for (u32 x = t + tid; x < e; x += kThreads) {
         const u32 first = (x - tile_base) * kTile<B>;
@@ -976,12 +980,12 @@ __device__ void plan_segment(const Sort<B>& a, Segment* seg, const Map<B>& m, co
     if (n <= kWideCap<B>) {  // what 512 threads sort in one block: the tail does it
       a.crowded[atomicAdd(&a.st->crowded, 1u)] = make_uint2(at0, n | (in ? kUnitSrc : 0u));
     } else if (identity || cell_is_one_value<B>(m, tab, sm.cell[i])) {
-      const u32 chunk = max(cap, (n + 255u) / 256u), chunks = (n + chunk - 1) / chunk;
+      const u32 chunk = max(cap, parts_of(n, 256u)), chunks = parts_of(n, chunk);
       const u32 u = atomicAdd(&a.st->units, chunks);
       for (u32 x = 0; x < chunks; ++x)
         a.units[u + x] = make_uint2(at0 + x * chunk, min(chunk, n - x * chunk) | (in ? kUnitSrc : 0u) | kUnitCopy);
     } else {
-      const u32 tiles = (n + kTile<B> - 1) / kTile<B>;
+      const u32 tiles = parts_of(n, kTile<B>);
       const u64 got = atomicAdd(&a.st->list[to], (u64(1) << 32) | tiles);
       const u32 id = u32(got >> 32), tb = u32(got);
       Segment* o = a.segs(to) + id;
@@ -1010,7 +1014,7 @@ template <typename B>
 __device__ void plan_zeros(const Sort<B>& a, u32* tmp) {
   const u32 neg = __ldcg(&a.st->neg_zeros), pos = __ldcg(&a.st->pos_zeros);
   if (neg == 0 || pos == 0) return;
-  const u32 tiles = (a.n + kTile<B> - 1) / kTile<B>;
+  const u32 tiles = parts_of(a.n, kTile<B>);
   const u32 words = u32((u64(neg) + pos + 31) / 32);
   for (u32 i = threadIdx.x; i < words; i += kThreads) a.zero_signs[i] = 0u;
   u32 carry = 0;
@@ -1052,7 +1056,7 @@ template <typename B, int KIND>
 __global__ __launch_bounds__(kThreads, 2) void part_histogram_root_kernel(Sort<B> a) {
   __shared__ HistSmem<B> sm;
   __shared__ PlanSmem plan;
-  const u32 tiles = (a.n + kTile<B> - 1) / kTile<B>;
+  const u32 tiles = parts_of(a.n, kTile<B>);
   const u32 t0 = u32(u64(tiles) * blockIdx.x / gridDim.x), t1 = u32(u64(tiles) * (blockIdx.x + 1) / gridDim.x);
   histogram_tiles<B, KIND, true>(a, a.segs(0), 1u, a.count0, t0, t1, sm);
   __threadfence();
@@ -1104,7 +1108,7 @@ __global__ __launch_bounds__(1024) void part_segments_kernel(Sort<B> a, const u6
       first = u32(offsets[id]);
       len = u32(offsets[id + 1u] - offsets[id]);
     }
-    const u32 tiles = (len + kTile<B> - 1) / kTile<B>;
+    const u32 tiles = parts_of(len, kTile<B>);
     u32 total;
     const u32 at = base + block_scan<1024>(tiles, tmp, &total);
     const bool ok = i < segs && at + tiles <= max_tiles;
@@ -1128,7 +1132,7 @@ __global__ __launch_bounds__(1024) void part_segments_kernel(Sort<B> a, const u6
   if (threadIdx.x == 0) {
     if (taken) {
       const u32 id = ids[taken - 1u];
-      const u32 tiles = (u32(offsets[id + 1u] - offsets[id]) + kTile<B> - 1) / kTile<B>;
+      const u32 tiles = parts_of(u32(offsets[id + 1u] - offsets[id]), kTile<B>);
       a.st->list[1] = (u64(taken) << 32) | (a.seg1[taken - 1u].tile_base + tiles);
     }
     if (!fits && a.status != nullptr) atomicOr(a.status, kStatusBadInput);
@@ -1349,7 +1353,7 @@ __global__ __launch_bounds__(kThreads, Shape<sizeof(B)>::kTileBlocks) void part_
   ScatterSmem<B>& sm = *reinterpret_cast<ScatterSmem<B>*>(smem_raw);
   const Segment* segs = a.segs(ROOT ? 0u : 1u);
   if (ROOT && __ldcg(&segs->identity)) return;
-  const u32 tiles = ROOT ? (a.n + kTile<B> - 1) / kTile<B> : u32(__ldcg(&a.st->list[1]));
+  const u32 tiles = ROOT ? parts_of(a.n, kTile<B>) : u32(__ldcg(&a.st->list[1]));
   const u32 t0 = u32(u64(tiles) * blockIdx.x / gridDim.x), t1 = u32(u64(tiles) * (blockIdx.x + 1) / gridDim.x);
   scatter_tiles<B, KIND, ROOT>(a, segs, t0, t1, sm);
 }
@@ -2228,7 +2232,7 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
       if (!__ldcg(&seg->done) || __ldcg(&seg->src)) continue;
       B* p = a.keys + __ldcg(&seg->start);
       const u32 len = __ldcg(&seg->len);
-      for (u32 i = b * kThreads + tid; i < len; i += G * kThreads) p[i] = from_ordered<B, KIND>(__ldcg(p + i));
+      for (u64 i = b * kThreads + tid; i < len; i += G * kThreads) p[i] = from_ordered<B, KIND>(__ldcg(p + i));
     }
   }
   for (bool first = true; ok; first = false) {
@@ -2280,7 +2284,7 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
       constexpr B sign = B(1) << (sizeof(B) * 8 - 1);
       const u32 lo = __ldcg(&a.st->below_zeros);
       const u32 zeros = neg + pos;
-      for (u32 i = b * kThreads + tid; i < zeros; i += G * kThreads)
+      for (u64 i = b * kThreads + tid; i < zeros; i += G * kThreads)  // 64 bits: a step past 2^32 must not wrap
         a.keys[lo + i] = !pos || ((__ldcg(a.zero_signs + (i >> 5)) >> (i & 31u)) & 1u) ? sign : B(0);
     }
   }

@@ -75,3 +75,51 @@ def test_heavy_end_values_in_large_segments_match_oracle(ctx, orc, dtype):
     ctx.segmented_sort_device(t.data_ptr(), a.size, o.data_ptr(), len(parts), NAMES[dtype])
     ctx.synchronize()
     assert t.cpu().numpy().view(dtype).tobytes() == orc.segmented_sort(a, offs).tobytes()
+
+
+LARGEST = (1 << 32) - 1  # the most keys a sort takes
+STEP = 1 << 28
+
+
+def sort_largest(ctx, fill, dtype):
+    """LARGEST 4-byte keys, made and sorted in place on the device; fill(i) gives the keys at positions i."""
+    temp_bytes = ctx.sort_temp_bytes(dtype, LARGEST)
+    if torch.cuda.mem_get_info()[0] < 4 * LARGEST + temp_bytes + (16 << 30):
+        pytest.skip("not enough device memory")
+    t = torch.empty(LARGEST, dtype=torch.int32, device="cuda")
+    temp = torch.empty(temp_bytes, dtype=torch.uint8, device="cuda")
+    for i in range(0, LARGEST, STEP):
+        j = min(LARGEST, i + STEP)
+        t[i:j] = fill(torch.arange(i, j, device="cuda"))
+    torch.cuda.synchronize()
+    ctx.sort_device(t.data_ptr(), LARGEST, dtype, temp.data_ptr(), temp_bytes)
+    ctx.synchronize()
+    return t
+
+
+def check_largest(t, expected):
+    for i in range(0, LARGEST, STEP):
+        j = min(LARGEST, i + STEP)
+        assert torch.equal(t[i:j], expected(torch.arange(i, j, device="cuda"))), f"[{i}, {j})"
+
+
+def test_largest_sort_of_distinct_keys(ctx):
+    """Every uint32 but one, shuffled by an odd multiplier: the counts of tiles and chunks take nearly all 32 bits."""
+    missing = LARGEST * 2654435761 % (1 << 32)
+    t = sort_largest(ctx, lambda i: (i * 2654435761).to(torch.int32), "u32")
+    check_largest(t, lambda i: (i + (i >= missing)).to(torch.int32))
+
+
+def test_largest_sort_of_one_value_and_a_few_others(ctx):
+    """One value all but 4096 times: its cell is copied in chunks."""
+    t = sort_largest(ctx, lambda i: torch.where(i % (1 << 20) == 5, i >> 20, 5000).to(torch.int32), "u32")
+    check_largest(t, lambda i: torch.where(i < 4096, i, 5000).to(torch.int32))
+
+
+def test_largest_sort_of_zeros_of_both_signs(ctx):
+    """Zeros of both signs all but 15 times: their signs are written back in input order, over nearly all positions."""
+    sign, one = -(1 << 31), 0x3F800000
+    zero = lambda i: torch.where(i % 3 == 0, sign, 0)
+    t = sort_largest(ctx, lambda i: torch.where(i % STEP == STEP - 1, one, zero(i)).to(torch.int32), "f32")
+    others = LARGEST // STEP  # the input position of the i-th zero is i plus the others before it
+    check_largest(t, lambda i: torch.where(i >= LARGEST - others, one, zero(i + i // (STEP - 1))).to(torch.int32))

@@ -174,7 +174,9 @@ int mgs_kway_merge_device(mgs_ctx* ctx, int dtype, const void* const* d_runs, co
  * through the partition sort (integer keys) or the onesweep passes (IEEE keys)
  * all at once. The launch sequence does not read anything back to the host (stream-ordered, capturable in a CUDA graph).
  * Invalid offsets (decreasing, or beyond n) leave that segment unsorted and
- * make the next mgs_ctx_synchronize return MGS_ERR_INVALID. Asynchronous. */
+ * make the next mgs_ctx_synchronize return MGS_ERR_INVALID; so does a segment
+ * that overlaps an earlier one (only decreasing offsets make one), whose keys
+ * are then those of either or of neither sorted. Asynchronous. */
 int mgs_segmented_sort_temp_bytes(int dtype, size_t n, size_t num_segments, size_t* bytes);
 int mgs_segmented_sort_device(mgs_ctx* ctx, int dtype, void* d_keys, size_t n, const uint64_t* d_offsets,
                               size_t num_segments, void* d_temp, size_t temp_bytes, void* stream);

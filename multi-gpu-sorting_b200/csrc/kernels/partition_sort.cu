@@ -1090,16 +1090,16 @@ __global__ __launch_bounds__(kThreads) void part_map_kernel(Sort<B> a) {
 }
 
 // Segmented sort: its large segments as list 1. One block, 1024 segments a
-// round. Segments that do not fit the scratch (they overlap: the offsets are out
-// of order) are left out and reported.
+// round. A segment that starts before the end of an earlier large one (the
+// offsets are out of order) is left out and reported: disjoint segments of the
+// array are what the lists' capacities are computed for (layout).
 template <typename B>
 __global__ __launch_bounds__(1024) void part_segments_kernel(Sort<B> a, const u64* __restrict__ offsets,
-                                                             const u32* __restrict__ ids, const u32* __restrict__ count,
-                                                             u32 max_segs, u32 max_tiles) {
-  __shared__ u32 tmp[33];
-  const u32 all = *count, segs = min(all, max_segs);
-  u32 taken = 0, base = 0;
-  bool fits = all <= max_segs;
+                                                             const u32* __restrict__ ids, const u32* __restrict__ count) {
+  __shared__ u32 tmp[33], last_end[32];
+  const u32 segs = *count, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  u32 taken = 0, base = 0, end = 0;  // of the rounds so far: segments and tiles in the list, the largest end
+  bool left_out = false;
   for (u32 r = 0; r < segs; r += 1024u) {
     const u32 i = r + threadIdx.x;
     u32 first = 0, len = 0;
@@ -1108,35 +1108,41 @@ __global__ __launch_bounds__(1024) void part_segments_kernel(Sort<B> a, const u6
       first = u32(offsets[id]);
       len = u32(offsets[id + 1u] - offsets[id]);
     }
+    u32 reach = first + len;  // the largest end up to this segment
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 t = __shfl_up_sync(0xffffffffu, reach, o);
+      if (lane >= u32(o)) reach = max(reach, t);
+    }
+    if (lane == 31u) last_end[warp] = reach;
+    __syncthreads();
+    u32 before = __shfl_up_sync(0xffffffffu, reach, 1);  // ... up to the one before it
+    if (lane == 0) before = 0;
+    before = max(max(before, end), warp_max(lane < warp ? last_end[lane] : 0u));
+    end = max(end, warp_max(last_end[lane]));
+    const bool ok = i < segs && first >= before;
+    left_out |= i < segs && !ok;
     const u32 tiles = parts_of(len, kTile<B>);
+    // Segments and tiles in one scan: a round's disjoint segments have at most 2^20 full tiles and 1024 shorter ones.
+    static_assert(kTile<B> >= 4096u, "a round's tiles fit 21 bits");
     u32 total;
-    const u32 at = base + block_scan<1024>(tiles, tmp, &total);
-    const bool ok = i < segs && at + tiles <= max_tiles;
+    const u32 at = block_scan<1024>(ok ? (1u << 21) | tiles : 0u, tmp, &total);
     if (ok) {
+      const u32 id = taken + (at >> 21);
       Segment s;
       s.start = first;
       s.len = len;
-      s.tile_base = at;
-      s.cell_base = i * 8u + at * kCellsPerTile<B>;
+      s.tile_base = base + (at & ((1u << 21) - 1u));
+      s.cell_base = id * 8u + s.tile_base * kCellsPerTile<B>;
       s.src = s.identity = s.done = s.pad = 0u;
-      a.seg1[i] = s;
+      a.seg1[id] = s;
     }
-    const u32 n_ok = __syncthreads_count(ok);
-    taken += n_ok;
-    if (n_ok < min(1024u, segs - r)) {  // the first that did not fit ends the list: its tiles are not counted
-      fits = false;
-      break;
-    }
-    base += total;
+    taken += total >> 21;
+    base += total & ((1u << 21) - 1u);
+    __syncthreads();  // tmp and last_end are read
   }
-  if (threadIdx.x == 0) {
-    if (taken) {
-      const u32 id = ids[taken - 1u];
-      const u32 tiles = parts_of(u32(offsets[id + 1u] - offsets[id]), kTile<B>);
-      a.st->list[1] = (u64(taken) << 32) | (a.seg1[taken - 1u].tile_base + tiles);
-    }
-    if (!fits && a.status != nullptr) atomicOr(a.status, kStatusBadInput);
-  }
+  if (threadIdx.x == 0 && taken) a.st->list[1] = (u64(taken) << 32) | base;
+  if (__syncthreads_or(left_out) && threadIdx.x == 0 && a.status != nullptr) atomicOr(a.status, kStatusBadInput);
 }
 
 // Every segment of list 1.
@@ -2305,6 +2311,23 @@ struct Layout {
 };
 
 // Scratch for n keys; segments > 0: of a segmented sort with that many large segments at most.
+//
+// Capacities of the lists (the kernels append without a check). The segments of
+// a list are disjoint parts of the array, and a level's cells are disjoint
+// parts of its segments, because a segment's counts sum to its length (its
+// histogram counts every key once, whatever the keys are):
+//   segments: list 1 of a segmented sort has `segments` at most; every other
+//             segment has more than kWideCap keys, so n / (kWideCap + 1).
+//   tiles   : a full tile per kTile keys and a shorter one per segment.
+//   cells   : 8 per segment and kCellsPerTile per tile (see there).
+//   units   : with h = kCap / 2: a segment of len keys breaks into at most
+//             len / h windows, 2 runs more per cell above h, and 2 at its ends:
+//             3 len / h + 2 runs; cells of one value go in chunks of kCap keys or
+//             more, and one shorter one. Two levels before the units are sorted,
+//             on disjoint keys (a key of the second level has no unit of the
+//             first): 3 n / h + 2 segments of list 1 + 3 n / h + 2 n / kWideCap
+//             + n / kCap, below 8 n / h + 2 segments + 4096.
+//   crowded : units that were not in order, and runs of more than kCap keys.
 template <typename B, int KIND>
 Layout layout(size_t n, size_t segments) {
   Layout L{};
@@ -2480,7 +2503,7 @@ cudaError_t segments_typed(B* keys, size_t n, const u64* offsets, const u32* ids
   cudaError_t e = cudaMemsetAsync(tb, 0, L.clear_bytes, stream);
   if (e != cudaSuccess) return e;
   e = launch_kernel(rec, "part_segments", part_segments_kernel<B>, dim3(1), dim3(1024), 0, stream, a, offsets, ids,
-                    count, u32(max_count), u32(L.max_tiles));
+                    count);
   if (e != cudaSuccess) return e;
   e = launch_level<B, KIND>(a, std::min<size_t>(max_count, size_t(sms) * 4), true, sms, stream, rec);
   if (e != cudaSuccess) return e;

@@ -22,7 +22,8 @@ cudaError_t partition_sort(int dtype, void* d_keys, size_t n, void* d_temp, size
 // The large segments of a segmented sort of integer keys: segment ids[i], i <
 // *d_count <= max_segments, is [d_offsets[ids[i]], d_offsets[ids[i] + 1]) of
 // d_keys (all device arrays), of more than two blocks' worth of keys; each is
-// sorted on its own. (Not IEEE keys: the order of zeros of both signs is kept
+// sorted on its own. A segment that starts before an earlier one's end is left
+// as it is and reported (kStatusBadInput). (Not IEEE keys: the order of zeros of both signs is kept
 // for a whole array only.) Temp bytes 0 for IEEE types.
 size_t partition_segments_temp_bytes(int dtype, size_t n, size_t max_segments);
 cudaError_t partition_segments(int dtype, void* d_keys, size_t n, const unsigned long long* d_offsets,

@@ -123,3 +123,33 @@ def test_largest_sort_of_zeros_of_both_signs(ctx):
     t = sort_largest(ctx, lambda i: torch.where(i % STEP == STEP - 1, one, zero(i)).to(torch.int32), "f32")
     others = LARGEST // STEP  # the input position of the i-th zero is i plus the others before it
     check_largest(t, lambda i: torch.where(i >= LARGEST - others, one, zero(i + i // (STEP - 1))).to(torch.int32))
+
+
+@pytest.mark.parametrize("dtype", ["u4", "i8"])
+def test_overlapping_large_segments_are_left_out(ctx, mgs, orc, dtype):
+    """Offsets that go back make segments overlap. A large one that starts before an earlier one's end stays as it is
+    and is reported; the disjoint ones are sorted, and nothing is written behind the scratch."""
+    n = 1 << 20
+    rng = np.random.default_rng(6)
+    a = rng.integers(0, 1 << 31, n).astype(dtype)
+    q = n // 4
+    cases = [([0, 2 * q, q, 3 * q, n], [(0, 2 * q), (3 * q, n)]),
+             ([0, 3 * q, 0, 3 * q], [(0, 3 * q)]),
+             ([0, 3 * q] * 1500 + [3 * q, n], [(0, 3 * q), (3 * q, n)]),
+             ([q, 2 * q] + [0, q] * 3 + [2 * q, n], [(q, 2 * q), (2 * q, n)])]
+    for offs, kept in cases:
+        nseg = len(offs) - 1
+        temp_bytes = ctx.segmented_sort_temp_bytes(NAMES[dtype], n, nseg)
+        temp = torch.full((temp_bytes + (1 << 20),), 0x5A, dtype=torch.uint8, device="cuda")
+        t = torch.from_numpy(a.view(np.int32 if a.itemsize == 4 else np.int64).copy()).cuda()
+        o = torch.tensor(offs, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        ctx.segmented_sort_device(t.data_ptr(), n, o.data_ptr(), nseg, NAMES[dtype], temp.data_ptr(), temp_bytes)
+        with pytest.raises(mgs.MgsError) as e:
+            ctx.synchronize()
+        assert e.value.code == mgs.MGS_ERR_INVALID
+        want = a.copy()
+        for b, c in kept:
+            want[b:c] = orc.sort(a[b:c])
+        assert t.cpu().numpy().view(dtype).tobytes() == want.tobytes(), offs[:5]
+        assert bool((temp[temp_bytes:] == 0x5A).all())

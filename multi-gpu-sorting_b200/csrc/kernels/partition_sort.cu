@@ -678,14 +678,15 @@ __device__ Map<B> build_map(const B* __restrict__ src, u32 len, MapSmem<B>& sm, 
   block_scan<kThreads>(over, sm.tmp, &over);
   __syncthreads();
   if (over <= samples / 8u) return m;
-  // No: the quantiles of the (first keys of the) sample, sorted in the scratch.
+  // No: the quantiles of the sample, sorted in the scratch: of every second key where it does not hold them all
+  // (not of the first half: samples are in the order of the keys, which may be sorted).
   constexpr u32 kSorted = kHistWords * 4u / u32(sizeof(B));
   B* const sorted = reinterpret_cast<B*>(scratch);
-  const u32 count = min(samples, kSorted);  // powers of two both
+  const u32 count = min(samples, kSorted), every = samples / count;  // powers of two all
   __syncthreads();
 #pragma unroll
   for (u32 i = 0; i < kPer; ++i)
-    if (i * kThreads < count) sorted[i * kThreads + tid] = x[i];
+    if (i < per && (tid & (every - 1u)) == 0u) sorted[(i * kThreads + tid) / every] = x[i];
   for (u32 size = 2; size <= count; size <<= 1) {
     for (u32 d = size >> 1; d > 0; d >>= 1) {
       __syncthreads();

@@ -153,3 +153,19 @@ def test_overlapping_large_segments_are_left_out(ctx, mgs, orc, dtype):
             want[b:c] = orc.sort(a[b:c])
         assert t.cpu().numpy().view(dtype).tobytes() == want.tobytes(), offs[:5]
         assert bool((temp[temp_bytes:] == 0x5A).all())
+
+
+@pytest.mark.parametrize("dtype", ["u8", "i8", "f8"])
+def test_ordered_clustered_keys_match_oracle(ctx, orc, dtype):
+    """Sorted, reversed and nearly sorted keys whose cells are quantiles of the sample (clusters, heavy tails)."""
+    n = 1_500_000
+    rng = np.random.default_rng(7)
+    clusters = np.sort(rng.integers(0, 1 << 62, 2000))[rng.integers(0, 2000, n)] + rng.integers(0, 3000, n)
+    tail = (np.maximum(rng.random(n), 1e-6) ** -5).astype(np.int64) << 8
+    for a in (np.sort(clusters), np.sort(tail)):
+        nearly = a.copy()
+        i = rng.permutation(n)[:n // 50]
+        nearly[i] = nearly[rng.permutation(i)]
+        for b in (a, a[::-1], nearly):
+            b = np.ascontiguousarray(b).view(dtype)
+            assert sorted_on_device(ctx, b).tobytes() == orc.sort(b).tobytes()

@@ -18,7 +18,8 @@
 //                       cells) in shared memory and stores it to the caller's
 //                       buffer.
 //   P4 part_tail      : one cooperative launch for the rest, mostly nothing:
-//                       units whose keys sit crowded, cells that hold one value,
+//                       units that the common way left out of order or that are
+//                       too large for it, cells that hold one value,
 //                       and, through the same steps once more, cells that two
 //                       levels left too large (keys clustered at several
 //                       scales); the zeros' signs; the status.
@@ -69,8 +70,8 @@ constexpr u32 kBarrierSpins = 1u << 25;
 // thread's consecutive keys free of bank conflicts. Small blocks, because the
 // steps of a unit are short and separated by barriers: 2^28 uint32, part_local
 // with 512 x 20 keys and two blocks per SM 1.39 ms, 256 x 28 and three 1.37 ms,
-// 384 x 20 and three 1.39 ms, 256 x 20 and four 1.27 ms (same code, before the
-// call on crowded bins was moved out of it).
+// 384 x 20 and three 1.39 ms, 256 x 20 and four 1.27 ms (same code, with a
+// call for crowded bins in it).
 // kTileItems keys per thread make a scatter tile, kTileBlocks blocks per SM: a
 // larger tile has longer runs per cell and fewer global atomics per key, until
 // its keys spill. 2^28 uint32, both scatters: 16 items and two blocks 1.43 ms,
@@ -334,7 +335,7 @@ struct alignas(16) Segment {
 
 struct State {
   u64 list[2];        // per segment list: segments << 32 | tiles
-  u32 units, next_unit, crowded;
+  u32 units, next_unit, left;
   u32 hist_done;
   u32 error;
   u32 neg_zeros, pos_zeros, below_zeros;  // IEEE keys: -0.0, +0.0, keys that sort before them
@@ -363,7 +364,7 @@ struct Sort {
   MapTable<B>* tables;  // likewise
   uint4* tiles;    // per tile of a list: first key, keys, segment, buffer
   uint2* units;
-  uint2* crowded;  // units left by the common way
+  uint2* left;  // units for the tail: of more than kCap keys, or not in order after the common way
   u32* tile_zeros;  // root tiles: zeros of both signs; then their exclusive prefix
   u32* zero_signs;  // bit i: the i-th zero of the input is -0.0
   u32* status;
@@ -382,8 +383,6 @@ __device__ __forceinline__ Map<B> load_map(const Map<B>* p) {
 }
 
 // ---------------------------------------------------------------- blocks ----
-__device__ __forceinline__ u32 lane_of() { return threadIdx.x & 31u; }
-
 // Exclusive scan over the block (any multiple of 32 threads up to 1024); total
 // out. Ends without a barrier after the last read of `tmp`: callers separate
 // uses with a barrier of their own.
@@ -634,7 +633,10 @@ __device__ Map<B> build_map(const B* __restrict__ src, u32 len, MapSmem<B>& sm, 
       m = equal;
     }
   }
-  u32 ni = inner_cells<B>(len, kCellSampled<B>, 2u);
+  const u32 want = inner_cells<B>(len, kCellSampled<B>, 2u);
+  // Twice as many where one level has room for them: fewer cells are then above a unit, which only the tail sorts
+  // (neighbouring small cells make a unit together). 10^6 normal float32 with 0.1 % zeros and NaN: 97 -> 79 us.
+  u32 ni = len <= kOneLevel<B> ? min(2u * want, kMaxCells - 2u) : want;
   m.ncells = ni + 2u;
   {
     const u64 all = u64(ni) << kFixBits;
@@ -671,7 +673,7 @@ __device__ Map<B> build_map(const B* __restrict__ src, u32 len, MapSmem<B>& sm, 
   __syncthreads();
   const bool last_level = len <= kOneLevel<B>;
   const u32 most =
-      last_level ? 3u * samples / ni + 8u : u32(0.6f * float(kMaxCells) * float(kCellSampled<B>) * float(samples) / float(len)) + 8u;
+      last_level ? 3u * samples / want + 8u : u32(0.6f * float(kMaxCells) * float(kCellSampled<B>) * float(samples) / float(len)) + 8u;
   u32 over = 0;
   for (u32 q = tid; q < m.ncells; q += kThreads)
     if (cell_count[q] > most && cell_min[q] != cell_max[q]) over += cell_count[q];
@@ -701,7 +703,7 @@ __device__ Map<B> build_map(const B* __restrict__ src, u32 len, MapSmem<B>& sm, 
     }
   }
   __syncthreads();
-  ni = min(2u * ni, kMaxCells - 2u);  // quantiles of a sample are rough: more of them
+  ni = min(2u * want, kMaxCells - 2u);  // quantiles of a sample are rough: more of them
   m.kind = kSplit;
   m.ncells = ni + 1u;  // edges: the smallest key, then ni - 1 quantiles
   m.scale = 1u << (31u - u32(__clz(int(ni))));
@@ -810,6 +812,20 @@ __device__ __noinline__ ZeroCounts count_range(const B* __restrict__ p, u32 n, c
   return z;
 }
 
+// The segment of a tile: the largest s with tile_base <= t.
+__device__ __forceinline__ u32 segment_of(const Segment* segs, u32 nseg, u32 t) {
+  u32 s = 0, hi = nseg;
+  while (hi - s > 1u) {
+    const u32 mid = (s + hi) / 2u;
+    if (__ldcg(&segs[mid].tile_base) <= t) {
+      s = mid;
+    } else {
+      hi = mid;
+    }
+  }
+  return s;
+}
+
 // Counts the cells of the tiles [t0, t1) of a segment list into counts. The
 // segments' maps are ready.
 template <typename B, int KIND, bool ROOT>
@@ -817,16 +833,7 @@ __device__ void histogram_tiles(const Sort<B>& a, const Segment* segs, u32 nseg,
                                 HistSmem<B>& sm) {
   const u32 tid = threadIdx.x;
   if (t0 >= t1) return;
-  u32 s = 0;  // the segment of tile t0: the largest s with tile_base <= t0
-  u32 hi = ROOT ? 1u : nseg;
-  while (hi - s > 1) {
-    const u32 mid = (s + hi) / 2;
-    if (__ldcg(&segs[mid].tile_base) <= t0) {
-      s = mid;
-    } else {
-      hi = mid;
-    }
-  }
+  u32 s = segment_of(segs, ROOT ? 1u : nseg, t0);
   ZeroCounts z{0, 0, 0};
   for (u32 t = t0; t < t1; ++s) {
     const uint4 head = ROOT ? make_uint4(0u, a.n, 0u, 0u) : __ldcg(reinterpret_cast<const uint4*>(segs + s));
@@ -979,7 +986,7 @@ __device__ void plan_segment(const Sort<B>& a, Segment* seg, const Map<B>& m, co
     }
     const u32 at0 = start + sm.start[i];
     if (n <= kWideCap<B>) {  // what 512 threads sort in one block: the tail does it
-      a.crowded[atomicAdd(&a.st->crowded, 1u)] = make_uint2(at0, n | (in ? kUnitSrc : 0u));
+      a.left[atomicAdd(&a.st->left, 1u)] = make_uint2(at0, n | (in ? kUnitSrc : 0u));
     } else if (identity || cell_is_one_value<B>(m, tab, sm.cell[i])) {
       const u32 chunk = max(cap, parts_of(n, 256u)), chunks = parts_of(n, chunk);
       const u32 u = atomicAdd(&a.st->units, chunks);
@@ -1204,7 +1211,7 @@ __device__ __forceinline__ void load_tile(B (&k)[Shape<sizeof(B)>::kTileItems], 
 template <typename B, int KIND, bool ROOT, bool WHOLE, u32 MAP, u32 X>
 __device__ __forceinline__ void scatter_tile(const Sort<B>& a, B (&k)[Shape<sizeof(B)>::kTileItems],
                                              B* __restrict__ dst, u32 cnt, const B* __restrict__ next, u32 next_cnt,
-                                             u32 tile, u32 which, ScatterSmem<B>& sm) {
+                                             u32 tile, bool signs, u32 which, ScatterSmem<B>& sm) {
   constexpr int kItems = Shape<sizeof(B)>::kTileItems;
   const u32 tid = threadIdx.x;
   const int left = int(cnt) - int(tid);
@@ -1213,6 +1220,8 @@ __device__ __forceinline__ void scatter_tile(const Sort<B>& a, B (&k)[Shape<size
   u32* const counters = sm.cnt[which];
   unsigned char* const cnt_bytes = reinterpret_cast<unsigned char*>(counters);
   unsigned char* const key_bytes = reinterpret_cast<unsigned char*>(sm.keys);
+  u32 zeros_before = 0;
+  if (ROOT && KIND == kFloatKey && signs) zeros_before = __ldcg(a.tile_zeros + tile);  // on its way meanwhile
   u32 pk[kItems];  // the key's counter (byte offset) | its rank there << 16
   u32 neg_mask = 0;  // the items that are -0.0
   if (KIND != kUnsignedKey) {
@@ -1236,8 +1245,7 @@ __device__ __forceinline__ void scatter_tile(const Sort<B>& a, B (&k)[Shape<size
   }
   if (ROOT && KIND == kFloatKey) {
     // Signs of the zeros, in input order (item, then thread).
-    const u32 neg = __ldcg(&a.st->neg_zeros), pos = __ldcg(&a.st->pos_zeros);
-    if (neg && pos) {
+    if (signs) {
       static_assert(kItems * kWarps <= kThreads, "a count per warp and item");
       u32 zero_mask = 0;
 #pragma unroll
@@ -1252,7 +1260,7 @@ __device__ __forceinline__ void scatter_tile(const Sort<B>& a, B (&k)[Shape<size
       const u32 count = tid < kItems * kWarps ? sm.zeros[tid] : 0u;
       const u32 before = block_scan<kThreads>(count, sm.tmp, &total);
       if (total) {  // the same in every thread
-        if (tid < kItems * kWarps) sm.zeros[tid] = __ldcg(a.tile_zeros + tile) + before;
+        if (tid < kItems * kWarps) sm.zeros[tid] = zeros_before + before;
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < kItems; ++i) {
@@ -1319,6 +1327,7 @@ __device__ void scatter_tiles(const Sort<B>& a, const Segment* segs, u32 t0, u32
   uint4 cur = tile_at(t0);
   load_tile<B>(k, a.buf(cur.w) + cur.x, cur.y);
   u32 have = ~0u, which = 0;
+  const bool signs = ROOT && KIND == kFloatKey && __ldcg(&a.st->neg_zeros) && __ldcg(&a.st->pos_zeros);
   reinterpret_cast<uint4*>(sm.cnt[0])[tid] = make_uint4(0u, 0u, 0u, 0u);
   for (u32 t = t0; t < t1; ++t) {
     uint4 next = cur;
@@ -1343,9 +1352,9 @@ __device__ void scatter_tiles(const Sort<B>& a, const Segment* segs, u32 t0, u32
       with_kind<B>(sm.map, [&](auto kind, auto x) {
         constexpr u32 kKind = decltype(kind)::value, kX = decltype(x)::value;
         if (cur.y == kTile<B>) {
-          scatter_tile<B, KIND, ROOT, true, kKind, kX>(a, k, dst, cur.y, ahead, next.y, t, which, sm);
+          scatter_tile<B, KIND, ROOT, true, kKind, kX>(a, k, dst, cur.y, ahead, next.y, t, signs, which, sm);
         } else {
-          scatter_tile<B, KIND, ROOT, false, kKind, kX>(a, k, dst, cur.y, ahead, next.y, t, which, sm);
+          scatter_tile<B, KIND, ROOT, false, kKind, kX>(a, k, dst, cur.y, ahead, next.y, t, signs, which, sm);
         }
       });
       which ^= 1u;
@@ -1370,19 +1379,18 @@ __global__ __launch_bounds__(kThreads, Shape<sizeof(B)>::kTileBlocks) void part_
 // one bin per key; a key's place is its bin's start plus the rank that the
 // counting atomic returned. If a bin holds more than kBinLimit keys, the bins
 // are cut once more, each into as many parts as it holds keys, which evens out
-// any density that is smooth within a bin. Parts that are still crowded go
-// through the same steps by themselves, with their own range (the large ones),
-// or are sorted by a warp, unless they are in order, as equal keys are. Then every bin is at most kBinLimit long
-// or in order, and odd-even transposition in registers over each thread's
-// consecutive keys, and over windows across the threads' borders, finishes the
-// order: as many rounds as the fullest bin has keys.
+// any density that is smooth within a bin. Then every bin or part is mostly at
+// most kBinLimit long, and odd-even transposition in registers over each
+// thread's consecutive keys, and over windows across the threads' borders,
+// finishes the order: as many rounds as the fullest bin has keys. What is still
+// out of order after that (keys clustered at several scales) is merge sorted:
+// the same cost whatever the keys are.
 template <typename B>
 constexpr u32 kBinLimit = sizeof(B) == 4 ? 8 : 7;
 // Keys on either side of a border between two threads' keys that a bin across it can reach (a multiple of 16
 // bytes; the windows of neighbouring borders must not overlap).
 template <typename B>
 constexpr u32 kBorder = sizeof(B) == 4 ? 8 : 6;
-constexpr u32 kWarpPart = 256;  // crowded parts up to this size are sorted by a warp
 constexpr u32 kExactBits = 15;  // Bins gives every value a bin of its own for ranges below 2^kExactBits
 
 template <typename B, int THREADS, int ITEMS>
@@ -1390,14 +1398,11 @@ struct LocalSmem {
   static constexpr u32 kKeys = u32(THREADS) * ITEMS;
   static constexpr u32 kBins = u32(ITEMS + 3) / 4u * 4u * THREADS;  // a bin per key
   static_assert(kBins <= 1u << kExactBits, "a range below the bins' number must fit the exact bins");
-  static constexpr u32 kParts = kKeys / (kBinLimit<B> + 1) + 1, kBigParts = kKeys / (kWarpPart + 1) + 1;
   alignas(16) B keys[kKeys + 16];
   alignas(16) u32 bins[kBins + 4];
-  u32 part[kParts];  // start | keys << 16
-  u32 big_part[kBigParts];
   B mm[64];
   u32 tmp[4][33], most[33];
-  u32 parts, next, bigs, nbins;
+  u32 nbins;
 };
 
 // Exclusive scan in place of `groups` * 4 * THREADS counters (16-bit totals) in
@@ -1475,30 +1480,20 @@ __device__ __forceinline__ u32 scan_counters(u32* c, u32 groups, u32 (&tmp)[4][3
   return warp_max(lane < u32(THREADS / 32) ? most[lane] : 0u);
 }
 
-// Sorts keys[0..n) of shared memory with the lanes of a warp: Batcher's merge
-// exchange (Knuth, The Art of Computer Programming 3, 5.2.2, Algorithm M).
-template <typename B>
-__device__ void warp_network_sort(B* keys, u32 n, u32 lane) {
-  u32 top = 1;
-  while (top < n) top <<= 1;
-  for (u32 p = top >> 1; p > 0; p >>= 1) {
-    u32 q = top >> 1, r = 0, d = p;
-    for (;;) {
-      for (u32 i = lane; i + d < n; i += 32u) {
-        if ((i & p) == r) {
-          const B x = keys[i], y = keys[i + d];
-          if (y < x) {
-            keys[i] = y;
-            keys[i + d] = x;
-          }
-        }
-      }
-      __syncwarp();
-      if (q == p) break;
-      d = q - p;
-      q >>= 1;
-      r = p;
-    }
+// Two rounds of odd-even transposition over N registers.
+template <typename B, int N>
+__device__ __forceinline__ void transpose_twice(B (&x)[N]) {
+#pragma unroll
+  for (int i = 0; i + 1 < N; i += 2) {
+    const B lo = x[i] < x[i + 1] ? x[i] : x[i + 1], hi = x[i] < x[i + 1] ? x[i + 1] : x[i];
+    x[i] = lo;
+    x[i + 1] = hi;
+  }
+#pragma unroll
+  for (int i = 1; i + 1 < N; i += 2) {
+    const B lo = x[i] < x[i + 1] ? x[i] : x[i + 1], hi = x[i] < x[i + 1] ? x[i + 1] : x[i];
+    x[i] = lo;
+    x[i + 1] = hi;
   }
 }
 
@@ -1508,18 +1503,7 @@ __device__ __forceinline__ void transpose_rounds(B (&x)[N], u32 rounds) {
 #pragma unroll
   for (int r = 0; r < int(kBinLimit<B>); r += 2) {
     if (u32(r) >= rounds) break;
-#pragma unroll
-    for (int i = 0; i + 1 < N; i += 2) {
-      const B lo = x[i] < x[i + 1] ? x[i] : x[i + 1], hi = x[i] < x[i + 1] ? x[i + 1] : x[i];
-      x[i] = lo;
-      x[i + 1] = hi;
-    }
-#pragma unroll
-    for (int i = 1; i + 1 < N; i += 2) {
-      const B lo = x[i] < x[i + 1] ? x[i] : x[i + 1], hi = x[i] < x[i + 1] ? x[i + 1] : x[i];
-      x[i] = lo;
-      x[i + 1] = hi;
-    }
+    transpose_twice<B, N>(x);
   }
 }
 
@@ -1557,12 +1541,12 @@ __device__ __forceinline__ void store_run(B* p, const B (&x)[N]) {
 // The bins of one part of the keys: bin(key) = floor(offset * nbins / range),
 // the offset from the smallest key taken to 32 bits; one bin per value when
 // there are few enough values.
-template <typename B, bool MAY_LOG = false>
+template <typename B>
 struct Bins {
   B lo;
   u32 shift, mul, scale;
-  bool exact, log;
-  __device__ __forceinline__ Bins(B lo_, B range, u32 nbins, bool log_ = false) : lo(lo_), log(log_) {
+  bool exact;
+  __device__ __forceinline__ Bins(B lo_, B range, u32 nbins) : lo(lo_) {
     shift = 0;
     if constexpr (sizeof(B) == 8) {
       const int lz = leading_zeros(range);
@@ -1571,8 +1555,8 @@ struct Bins {
     exact = range < B(nbins);
     // Exact: d * 2^17 * 2^15 / 2^32 = d. Both products must fit: d < nbins <= 2^15 (checked in LocalSmem).
     mul = exact ? 1u << (32 - kExactBits) : 1u;
-    const u32 most = MAY_LOG && log ? log_x(range) : u32(range >> shift);
-    scale = exact ? 1u << kExactBits : u32(float(nbins) * (4294967296.f * 0.9999995f) / (float(most) + 1.f));
+    scale = exact ? 1u << kExactBits
+                  : u32(float(nbins) * (4294967296.f * 0.9999995f) / (float(u32(range >> shift)) + 1.f));
   }
   // bin in the high word, position within the bin (a 32-bit fraction) in the low word
   __device__ __forceinline__ u64 product(B key) const {
@@ -1582,162 +1566,9 @@ struct Bins {
     } else {
       dn = u32((key - lo) >> shift);
     }
-    if (MAY_LOG && log && !exact) {
-      dn = log_x(B(key - lo));
-    } else {
-      dn *= mul;
-    }
-    return u64(dn) * scale;
+    return u64(dn * mul) * scale;
   }
 };
-
-// Places keys whose bins are crowded: src[0..len) into sm.keys, in order up to
-// what the transposition rounds finish. Returns those rounds.
-template <typename B, int KIND, bool RAW, int THREADS, int ITEMS>
-__device__ __noinline__ u32 place_crowded(const B* src, u32 len, LocalSmem<B, THREADS, ITEMS>& sm) {
-  constexpr u32 kLimit = kBinLimit<B>;
-  constexpr u32 kGroup = 4u * THREADS;
-  constexpr int kFineGroups = (ITEMS + 3) / 4;
-  static_assert(kFineGroups * kGroup * 4 <= sizeof(sm.keys) - 4, "the finer counters lie over the keys");
-  const u32 tid = threadIdx.x;
-  B k[ITEMS];
-  u32 pk[ITEMS];
-  if (tid == 0) {
-    sm.parts = 0;
-    sm.next = 0;
-    sm.bigs = 0;
-  }
-  u32 base = 0, n = len;  // the part being placed
-  u32 rounds = 0;
-  for (bool first = true;; first = false) {
-    const int left = int(n) - int(tid);
-    B lo = ~B(0), hi = B(0);
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-      if (i * THREADS < left) {
-        if (first) {
-          k[i] = __ldcg(src + i * THREADS + tid);
-          if (RAW) k[i] = one_zero<B, KIND>(to_ordered<B, KIND>(k[i]));
-        } else {
-          k[i] = sm.keys[base + i * THREADS + tid];
-        }
-        lo = k[i] < lo ? k[i] : lo;
-        hi = k[i] > hi ? k[i] : hi;
-      }
-    }
-    const u32 groups = (n + kGroup - 1) / kGroup;
-    const u32 nbins = groups * kGroup;
-    for (u32 g = 0; g < groups; ++g) reinterpret_cast<uint4*>(sm.bins)[g * THREADS + tid] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid == 0) sm.bins[nbins] = n;  // the end of the last bin
-    block_min_max<THREADS, B>(lo, hi, sm.mm);
-    if (lo != hi) {
-      // Values crowded towards the smallest one: a third of the keys or more in the range's lowest 64th.
-      bool low = false;
-      if (first) {
-        u32 in_low = 0;
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) in_low += i * THREADS < left && (k[i] - lo) <= (hi - lo) / 64u ? 1u : 0u;
-        in_low = __reduce_add_sync(0xffffffffu, in_low);
-        u32 all;
-        block_scan<THREADS>(lane_of() == 0u ? in_low : 0u, sm.tmp[0], &all);
-        low = 3u * all >= n;
-        __syncthreads();
-      }
-      const Bins<B, true> bins(lo, hi - lo, nbins, low);
-#pragma unroll
-      for (int i = 0; i < ITEMS; ++i) {
-        if (i * THREADS < left) {
-          const u32 b = u32(bins.product(k[i]) >> 32);
-          pk[i] = b | (atomicAdd(&sm.bins[b], 1u) << 16);
-        }
-      }
-      __syncthreads();
-      u32 most = scan_counters<THREADS, kFineGroups>(sm.bins, groups, sm.tmp, sm.most);
-      if (bins.exact) most = 0;
-      const bool refine = first && most > kLimit;
-      u32* const fine = reinterpret_cast<u32*>(sm.keys);
-      const u32 fine_groups = (n + kGroup - 1) / kGroup;
-      if (refine) {
-        for (u32 g = 0; g < fine_groups; ++g) reinterpret_cast<uint4*>(fine)[g * THREADS + tid] = make_uint4(0u, 0u, 0u, 0u);
-        if (tid == 0) fine[fine_groups * kGroup] = n;
-      }
-      __syncthreads();
-      if (refine) {
-        // Each bin [s, e) cut into e - s parts, numbered like the positions.
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) {
-          if (i * THREADS < left) {
-            const u32 b = pk[i] & 0xFFFFu;
-            const u32 s = sm.bins[b], e = sm.bins[b + 1u];
-            const u32 f = s + __umulhi(u32(bins.product(k[i])), e - s);
-            pk[i] = f | (atomicAdd(&fine[f], 1u) << 16);
-          }
-        }
-        __syncthreads();
-        most = scan_counters<THREADS, kFineGroups>(fine, fine_groups, sm.tmp, sm.most);
-        __syncthreads();
-      }
-      if (most > kLimit) {
-        const u32* const starts = refine ? fine : sm.bins;
-        const u32 count = refine ? fine_groups * kGroup : nbins;
-        for (u32 f = tid; f < count; f += THREADS) {
-          const u32 s = starts[f], m = starts[f + 1u] - s;
-          if (m > kLimit) sm.part[atomicAdd(&sm.parts, 1u)] = (base + s) | (m << 16);
-        }
-      }
-      rounds = max(rounds, min(most, kLimit));
-      if (refine) {
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i)
-          if (i * THREADS < left) pk[i] = fine[pk[i] & 0xFFFFu] + (pk[i] >> 16);
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i)
-          if (i * THREADS < left) sm.keys[pk[i]] = k[i];
-      } else {
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i)
-          if (i * THREADS < left) sm.keys[base + sm.bins[pk[i] & 0xFFFFu] + (pk[i] >> 16)] = k[i];
-      }
-    } else if (first) {
-#pragma unroll
-      for (int i = 0; i < ITEMS; ++i)
-        if (i * THREADS < left) sm.keys[i * THREADS + tid] = k[i];
-    }
-    __syncthreads();
-    // Crowded parts, a warp each: most hold equal keys. Small ones that do not are sorted, large ones come back.
-    const u32 parts = sm.parts, lane = tid & 31u;
-    if (parts) {
-      for (;;) {
-        u32 e = 0;
-        if (lane == 0) e = atomicAdd(&sm.next, 1u);
-        e = __shfl_sync(0xffffffffu, e, 0);
-        if (e >= parts) break;
-        const u32 part = sm.part[e];
-        B* p = sm.keys + (part & 0xFFFFu);
-        const u32 m = part >> 16;
-        bool bad = false;
-        for (u32 i = lane; i + 1 < m; i += 32) bad |= p[i + 1] < p[i];
-        if (!__any_sync(0xffffffffu, bad)) continue;
-        if (m <= kWarpPart) {
-          warp_network_sort<B>(p, m, lane);
-        } else if (lane == 0) {
-          sm.big_part[atomicAdd(&sm.bigs, 1u)] = part;
-        }
-      }
-      __syncthreads();
-      if (tid == 0) sm.parts = sm.next = 0;
-    }
-    const u32 bigs = sm.bigs;
-    if (bigs == 0) break;
-    const u32 part = sm.big_part[bigs - 1u];
-    __syncthreads();
-    if (tid == 0) sm.bigs = bigs - 1u;
-    base = part & 0xFFFFu;
-    n = part >> 16;
-  }
-  return rounds;
-}
 
 // Writes the zeros with their signs, in input order (src, the caller's bits, is
 // still unsorted), over the sorted zeros in sm.keys. Ends with a barrier.
@@ -1950,6 +1781,73 @@ __device__ __forceinline__ void finish_order(u32 n, u32 rounds, LocalSmem<B, THR
   }
 }
 
+// Merge sort of the n keys in shared memory: each thread's consecutive keys by
+// transposition in registers, then rounds of pairwise merges, a thread per ITEMS
+// consecutive outputs. Pairs that are in order already (most are: the bins came
+// out in order) are left as they are. Begins after and ends with a barrier.
+// Bound by the latency of shared memory (a chain of ITEMS reads per round). It
+// took the place of binning crowded parts again, one after the other, and of
+// networks of one warp, whose cost grew with the number of clusters. B200, whole
+// sorts of 2000 clusters of int64: 10^6 187 -> 150 us, 3 * 10^6 310 -> 240,
+// 10^7 724 -> 554.
+template <typename B, int THREADS, int ITEMS>
+__device__ __forceinline__ void merge_order(u32 n, LocalSmem<B, THREADS, ITEMS>& sm) {
+  const u32 at = threadIdx.x * u32(ITEMS);
+  B x[ITEMS];
+  if (at < n) {
+    load_run<B, ITEMS>(sm.keys + at, x);
+#pragma unroll 1
+    for (int r = 0; r < ITEMS; r += 2) transpose_twice<B, ITEMS>(x);
+    store_run<B, ITEMS>(sm.keys + at, x);  // what lies after the last key sorts last (finish_order)
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (u32 w = ITEMS; w < n; w *= 2u) {  // runs of w keys
+    const u32 a0 = at - at % (2u * w), b0 = a0 + w, b1 = min(b0 + w, n);
+    const bool merge = at < n && b0 < n && sm.keys[b0] < sm.keys[b0 - 1u];
+    if (merge) {
+      const u32 d = at - a0;  // outputs of this pair before this thread's
+      u32 lo = d > b1 - b0 ? d - (b1 - b0) : 0u, hi = min(d, w);  // how many of them are the first run's
+      while (lo < hi) {
+        const u32 mid = (lo + hi) / 2u;
+        if (sm.keys[b0 + (d - 1u - mid)] < sm.keys[a0 + mid]) {
+          hi = mid;
+        } else {
+          lo = mid + 1u;
+        }
+      }
+      u32 i = a0 + lo, j = b0 + (d - lo);
+      B u = sm.keys[i], v = sm.keys[j];
+#pragma unroll
+      for (int t = 0; t < ITEMS; ++t) {  // after the last output both runs are used up: the padding follows
+        const bool first = i < b0 && (j >= b1 || !(v < u));
+        x[t] = first ? u : v;
+        if (first) {
+          u = sm.keys[++i];
+        } else {
+          v = sm.keys[++j];
+        }
+      }
+    }
+    __syncthreads();
+    if (merge) store_run<B, ITEMS>(sm.keys + at, x);
+    __syncthreads();
+  }
+}
+
+// Whether the keys are in order after finish_order and, when a bin held more
+// than kBinLimit keys, a few more of its rounds: they do for bins that are only
+// a little too full. merge_order is for the others.
+template <typename B, int THREADS, int ITEMS>
+__device__ __forceinline__ bool finished(u32 n, u32 rounds, LocalSmem<B, THREADS, ITEMS>& sm) {
+  if (rounds <= kBinLimit<B>) return true;
+  for (u32 tries = 0; !in_order<B, THREADS, ITEMS>(n, sm); ++tries) {
+    if (tries == 2u) return false;
+    finish_order<B, THREADS, ITEMS>(n, rounds, sm);
+  }
+  return true;
+}
+
 template <typename B, int KIND, int THREADS, int ITEMS>
 __device__ __forceinline__ void store_unit(B* __restrict__ dst, u32 n, LocalSmem<B, THREADS, ITEMS>& sm) {
   dst += threadIdx.x;
@@ -1967,9 +1865,9 @@ __device__ __forceinline__ const B* unit_keys(const Sort<B>& a, uint2 unit) {
 __device__ __forceinline__ u32 unit_load(uint2 unit) { return (unit.y & kUnitCopy) ? 0u : unit.y & kUnitLen; }
 
 // A unit whose keys are in k. ahead() runs once k is no longer needed. False
-// when bins were crowded with different keys: nothing is stored then, and
-// sort_crowded_unit has to do the unit (apart, because its call in the common
-// way costs a third more shared-memory traffic in spilled registers).
+// when bins were crowded with different keys: nothing is stored then, and the
+// keys are left in shared memory, not in order (merge_order is not called here,
+// because in part_local's loop it costs registers that the common way needs).
 template <typename B, int KIND, int THREADS, int ITEMS, class Ahead>
 __device__ __forceinline__ bool sort_unit(const Sort<B>& a, uint2 unit, const B (&k)[ITEMS],
                                           LocalSmem<B, THREADS, ITEMS>& sm, Ahead&& ahead) {
@@ -1991,22 +1889,27 @@ __device__ __forceinline__ bool sort_unit(const Sort<B>& a, uint2 unit, const B 
   }
   ahead();
   finish_order<B, THREADS, ITEMS>(len, rounds, sm);
-  if (rounds > kBinLimit<B>) {  // a few more rounds do for bins that are only a little too full
-    for (u32 tries = 0; !in_order<B, THREADS, ITEMS>(len, sm); ++tries) {
-      if (tries == 2u) return false;
-      finish_order<B, THREADS, ITEMS>(len, rounds, sm);
-    }
-  }
+  if (!finished<B, THREADS, ITEMS>(len, rounds, sm)) return false;
   store_unit<B, KIND, THREADS, ITEMS>(dst, len, sm);
   return true;
 }
 
+// A unit by itself; crowded: the common way failed on it before. Not inlined: the tail calls it in three places.
 template <typename B, int KIND, int THREADS, int ITEMS>
-__device__ __forceinline__ void sort_crowded_unit(const Sort<B>& a, uint2 unit, LocalSmem<B, THREADS, ITEMS>& sm) {
+__device__ __noinline__ void sort_any_unit(const Sort<B>& a, uint2 unit, bool crowded, LocalSmem<B, THREADS, ITEMS>& sm) {
   const u32 len = unit.y & kUnitLen;
-  __syncthreads();
-  const u32 rounds = place_crowded<B, KIND, false, THREADS, ITEMS>(unit_keys(a, unit), len, sm);
-  finish_order<B, THREADS, ITEMS>(len, rounds, sm);
+  B k[ITEMS];
+  load_unit<B, THREADS, ITEMS>(k, unit_keys(a, unit), unit_load(unit));
+  __syncthreads();  // the last use of sm
+  if (crowded) {
+    const int left = int(len) - int(threadIdx.x);
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) sm.keys[i * THREADS + threadIdx.x] = i * THREADS < left ? k[i] : ~B(0);
+    __syncthreads();
+  } else if (sort_unit<B, KIND, THREADS, ITEMS>(a, unit, k, sm, [] {})) {
+    return;
+  }
+  merge_order<B, THREADS, ITEMS>(len, sm);
   store_unit<B, KIND, THREADS, ITEMS>(a.keys + unit.x, len, sm);
 }
 
@@ -2034,7 +1937,7 @@ __global__ __launch_bounds__(Shape<sizeof(B)>::kLocalThreads, Shape<sizeof(B)>::
       next = s_next[turn];
       load_unit<B, THREADS, ITEMS>(k, unit_keys(a, next), unit_load(next));
     });
-    if (!done && threadIdx.x == 0) a.crowded[atomicAdd(&a.st->crowded, 1u)] = cur;  // the tail's
+    if (!done && threadIdx.x == 0) a.left[atomicAdd(&a.st->left, 1u)] = cur;  // the tail's
     if (next.y == 0u) break;
     cur = next;
     __syncthreads();
@@ -2056,13 +1959,10 @@ __global__ __launch_bounds__(THREADS, 1) void part_small_kernel(B* keys, u32 n) 
     if (KIND == kFloatKey && u32(i * THREADS) + threadIdx.x < n) neg |= k[i] == kNegZero<B>;
     k[i] = one_zero<B, KIND>(k[i]);
   }
-  u32 rounds = place_keys<B, THREADS, ITEMS>(k, n, sm);
+  const u32 rounds = place_keys<B, THREADS, ITEMS>(k, n, sm);
   if (rounds == kOneValue) return;
   finish_order<B, THREADS, ITEMS>(n, rounds, sm);
-  if (rounds > kBinLimit<B> && !in_order<B, THREADS, ITEMS>(n, sm)) {
-    rounds = place_crowded<B, KIND, true, THREADS, ITEMS>(keys, n, sm);
-    finish_order<B, THREADS, ITEMS>(n, rounds, sm);
-  }
+  if (!finished<B, THREADS, ITEMS>(n, rounds, sm)) merge_order<B, THREADS, ITEMS>(n, sm);
   if (KIND == kFloatKey) {
     if (__syncthreads_or(neg)) order_zeros<B, KIND, THREADS, ITEMS>(keys, n, sm);
   }
@@ -2139,27 +2039,14 @@ __global__ __launch_bounds__(kThreads, 2) void kway_unit_tile_kernel(const B* co
   }
 #pragma unroll
   for (int t = 0; t < ITEMS; ++t) key[t] = to_ordered<B, KIND>(key[t]);
-  u32 rounds = place_keys<B, kThreads, ITEMS>(key, cnt, sm);
+  const u32 rounds = place_keys<B, kThreads, ITEMS>(key, cnt, sm);
   if (rounds == kOneValue) {
     const B one = from_ordered<B, KIND>(key[0]);
     for (u32 i = tid; i < cnt; i += kThreads) out[d0 + i] = one;
     return;
   }
   finish_order<B, kThreads, ITEMS>(cnt, rounds, sm);
-  if (rounds > kBinLimit<B>) {
-    bool done = in_order<B, kThreads, ITEMS>(cnt, sm);
-    for (u32 tries = 0; !done && tries < 2u; ++tries) {
-      finish_order<B, kThreads, ITEMS>(cnt, rounds, sm);
-      done = in_order<B, kThreads, ITEMS>(cnt, sm);
-    }
-    if (!done) {  // crowded bins: the staged keys go out as they are and come back through the output
-      store_unit<B, KIND, kThreads, ITEMS>(out + d0, cnt, sm);
-      __threadfence_block();
-      __syncthreads();
-      rounds = place_crowded<B, KIND, true, kThreads, ITEMS>(out + d0, cnt, sm);
-      finish_order<B, kThreads, ITEMS>(cnt, rounds, sm);
-    }
-  }
+  if (!finished<B, kThreads, ITEMS>(cnt, rounds, sm)) merge_order<B, kThreads, ITEMS>(cnt, sm);
   store_unit<B, KIND, kThreads, ITEMS>(out + d0, cnt, sm);
 }
 
@@ -2186,15 +2073,7 @@ __device__ void probe_segments(const Sort<B>& a) {
   const u64 list = __ldcg(&a.st->list[a.last_list]);
   const u32 nseg = u32(list >> 32), tiles = u32(list);
   for (u32 t = blockIdx.x; t < tiles; t += gridDim.x) {
-    u32 s = 0, hi = nseg;
-    while (hi - s > 1) {
-      const u32 mid = (s + hi) / 2;
-      if (__ldcg(&segs[mid].tile_base) <= t) {
-        s = mid;
-      } else {
-        hi = mid;
-      }
-    }
+    const u32 s = segment_of(segs, nseg, t);
     const u32 start = __ldcg(&segs[s].start), len = __ldcg(&segs[s].len), src = __ldcg(&segs[s].src);
     const u32 first = (t - __ldcg(&segs[s].tile_base)) * kTile<B>;
     const u32 cnt = min(kTile<B>, len - first);
@@ -2202,6 +2081,7 @@ __device__ void probe_segments(const Sort<B>& a) {
     const B key = __ldcg(p);
     if (__syncthreads_or(ld_volatile_u32(&segs[s].done) == 0u)) continue;
     bool other = false;
+#pragma unroll 4
     for (u32 i = threadIdx.x; i < cnt; i += kThreads) {
       other |= __ldcg(p + first + i) != key;
       if (src) a.keys[start + first + i] = from_ordered<B, KIND>(key);
@@ -2213,7 +2093,7 @@ __device__ void probe_segments(const Sort<B>& a) {
   }
 }
 
-// Cooperative launch. Sorts the units with crowded bins, then goes on with the
+// Cooperative launch. Sorts the units that are left, then goes on with the
 // segments of list `cur`, if any are left; last, the zeros' signs and the status.
 template <typename B, int KIND>
 __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 cur) {
@@ -2224,22 +2104,30 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
   u32 waits = 0;
   bool ok = true;
   constexpr int ITEMS = Shape<sizeof(B)>::kWideItems;
-  u32 crowded = __ldcg(&a.st->crowded);  // the list up to here is done
-  for (u32 u = b; u < crowded; u += G)
-    sort_crowded_unit<B, KIND, kThreads, ITEMS>(a, __ldcg(a.crowded + u), sm.local);
+  u32 left = __ldcg(&a.st->left);  // the list up to here is done
+  // From the last block on: the first ones probe, meanwhile.
+  for (u32 u = G - 1u - b; u < left; u += G) {
+    const uint2 unit = __ldcg(a.left + u);
+    sort_any_unit<B, KIND, kThreads, ITEMS>(a, unit, (unit.y & kUnitLen) <= kCap<B>, sm.local);
+  }
   if (__ldcg(&a.st->list[cur]) != 0u) {
     probe_segments<B, KIND>(a);
     ok = grid_barrier(a.st, ++waits * G);
   }
-  // Probed segments of one value that sit in the caller's buffer: to the caller's bits.
+  // Probed segments of one value that sit in the caller's buffer: to the caller's bits. Tile by tile: a loop over the
+  // segments in every block was a chain of dependent reads, 1.3 us per segment (27 segments, 3 * 10^6 float64 with a
+  // heavy tail: 240 -> 206 us).
   if (KIND != kUnsignedKey && ok) {
-    const u32 nseg = u32(__ldcg(&a.st->list[cur]) >> 32);
-    for (u32 s = 0; s < nseg; ++s) {
-      const Segment* seg = a.segs(cur) + s;
+    const Segment* segs = a.segs(cur);
+    const u64 list = __ldcg(&a.st->list[cur]);
+    for (u32 t = b; t < u32(list); t += G) {
+      const Segment* seg = segs + segment_of(segs, u32(list >> 32), t);
       if (!__ldcg(&seg->done) || __ldcg(&seg->src)) continue;
-      B* p = a.keys + __ldcg(&seg->start);
-      const u32 len = __ldcg(&seg->len);
-      for (u64 i = b * kThreads + tid; i < len; i += G * kThreads) p[i] = from_ordered<B, KIND>(__ldcg(p + i));
+      const u32 first = (t - __ldcg(&seg->tile_base)) * kTile<B>;
+      const u32 cnt = min(kTile<B>, __ldcg(&seg->len) - first);
+      B* p = a.keys + __ldcg(&seg->start) + first;
+#pragma unroll 4
+      for (u32 i = tid; i < cnt; i += kThreads) p[i] = from_ordered<B, KIND>(__ldcg(p + i));
     }
   }
   for (bool first = true; ok; first = false) {
@@ -2268,18 +2156,10 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
     scatter_tiles<B, kUnsignedKey, false>(a, a.segs(cur), t0, t1, sm.scatter);
     if (!(ok = grid_barrier(a.st, ++waits * G))) break;
     const u32 units = __ldcg(&a.st->units);
-    for (u32 u = b; u < units; u += G) {
-      const uint2 unit = __ldcg(a.units + u);
-      B k[ITEMS];
-      load_unit<B, kThreads, ITEMS>(k, unit_keys(a, unit), unit_load(unit));
-      __syncthreads();
-      if (!sort_unit<B, KIND, kThreads, ITEMS>(a, unit, k, sm.local, [] {}))
-        sort_crowded_unit<B, KIND, kThreads, ITEMS>(a, unit, sm.local);
-    }
-    const u32 wide = __ldcg(&a.st->crowded);
-    for (u32 u = crowded + b; u < wide; u += G)
-      sort_crowded_unit<B, KIND, kThreads, ITEMS>(a, __ldcg(a.crowded + u), sm.local);
-    crowded = wide;
+    for (u32 u = b; u < units; u += G) sort_any_unit<B, KIND, kThreads, ITEMS>(a, __ldcg(a.units + u), false, sm.local);
+    const u32 more = __ldcg(&a.st->left);
+    for (u32 u = left + b; u < more; u += G) sort_any_unit<B, KIND, kThreads, ITEMS>(a, __ldcg(a.left + u), false, sm.local);
+    left = more;
     cur ^= 1u;
     // The lists and units of this level are read before any block starts the next one's first step (the
     // next level's first barrier comes before its first write to them).
@@ -2287,10 +2167,11 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
   if (KIND == kFloatKey && ok) {
     const u32 neg = __ldcg(&a.st->neg_zeros), pos = __ldcg(&a.st->pos_zeros);
     if (neg && !__ldcg(&a.st->in_place)) {
-      if ((waits || crowded) && !grid_barrier(a.st, ++waits * G)) return;  // every key is in its place
+      if ((waits || left) && !grid_barrier(a.st, ++waits * G)) return;  // every key is in its place
       constexpr B sign = B(1) << (sizeof(B) * 8 - 1);
       const u32 lo = __ldcg(&a.st->below_zeros);
       const u32 zeros = neg + pos;
+#pragma unroll 4
       for (u64 i = b * kThreads + tid; i < zeros; i += G * kThreads)  // 64 bits: a step past 2^32 must not wrap
         a.keys[lo + i] = !pos || ((__ldcg(a.zero_signs + (i >> 5)) >> (i & 31u)) & 1u) ? sign : B(0);
     }
@@ -2305,7 +2186,7 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
 size_t align_up(size_t x, size_t to) { return (x + to - 1) / to * to; }
 
 struct Layout {
-  size_t segs_off[2], counts_off[2], cursor_off, maps_off, tables_off, tiles_off, units_off, crowded_off, zeros_off, signs_off, keys_off,
+  size_t segs_off[2], counts_off[2], cursor_off, maps_off, tables_off, tiles_off, units_off, left_off, zeros_off, signs_off, keys_off,
       total, clear_bytes;
   size_t max_segs, max_tiles;
   bool small, two_levels;
@@ -2328,7 +2209,8 @@ struct Layout {
 //             on disjoint keys (a key of the second level has no unit of the
 //             first): 3 n / h + 2 segments of list 1 + 3 n / h + 2 n / kWideCap
 //             + n / kCap, below 8 n / h + 2 segments + 4096.
-//   crowded : units that were not in order, and runs of more than kCap keys.
+//   left    : disjoint runs of more than kCap keys, and units; the list is not
+//             emptied between levels, whose keys are disjoint too.
 template <typename B, int KIND>
 Layout layout(size_t n, size_t segments) {
   Layout L{};
@@ -2357,7 +2239,7 @@ Layout layout(size_t n, size_t segments) {
   L.tables_off = take(L.max_segs * sizeof(MapTable<B>));
   L.tiles_off = take(L.max_tiles * sizeof(uint4));
   L.units_off = take((8 * (n / (kCap<B> / 2)) + 2 * segments + 4096) * sizeof(uint2));
-  L.crowded_off = take((8 * (n / (kCap<B> / 2)) + 2 * segments + 4096) * sizeof(uint2));
+  L.left_off = take((8 * (n / (kCap<B> / 2)) + 2 * segments + 4096) * sizeof(uint2));
   L.signs_off = KIND == kFloatKey ? take(n / 8 + 8) : 0;
   L.keys_off = take(n * sizeof(B));
   L.total = off;
@@ -2379,7 +2261,7 @@ Sort<B> make_sort(const Layout& L, B* keys, size_t n, char* tb, uint32_t* d_stat
   a.tables = reinterpret_cast<MapTable<B>*>(tb + L.tables_off);
   a.tiles = reinterpret_cast<uint4*>(tb + L.tiles_off);
   a.units = reinterpret_cast<uint2*>(tb + L.units_off);
-  a.crowded = reinterpret_cast<uint2*>(tb + L.crowded_off);
+  a.left = reinterpret_cast<uint2*>(tb + L.left_off);
   a.tile_zeros = reinterpret_cast<u32*>(tb + L.zeros_off);
   a.zero_signs = reinterpret_cast<u32*>(tb + L.signs_off);
   a.status = d_status;

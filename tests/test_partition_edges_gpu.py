@@ -161,7 +161,7 @@ def test_ordered_clustered_keys_match_oracle(ctx, orc, dtype):
     n = 1_500_000
     rng = np.random.default_rng(7)
     clusters = np.sort(rng.integers(0, 1 << 62, 2000))[rng.integers(0, 2000, n)] + rng.integers(0, 3000, n)
-    tail = (np.maximum(rng.random(n), 1e-6) ** -5).astype(np.int64) << 8
+    tail = (np.maximum(rng.random(n), 1e-6) ** -2.5).astype(np.int64) << 8
     for a in (np.sort(clusters), np.sort(tail)):
         nearly = a.copy()
         i = rng.permutation(n)[:n // 50]
@@ -169,3 +169,44 @@ def test_ordered_clustered_keys_match_oracle(ctx, orc, dtype):
         for b in (a, a[::-1], nearly):
             b = np.ascontiguousarray(b).view(dtype)
             assert sorted_on_device(ctx, b).tobytes() == orc.sort(b).tobytes()
+
+
+def several_scales(dtype, n, rng):
+    """Keys in clusters within clusters: bins and parts of bins hold many different keys, and merges order them."""
+    bits = 8 * np.dtype(dtype).itemsize
+    top = rng.integers(0, 1 << (bits - 1), 5, dtype=np.uint64)[rng.integers(0, 5, n)]
+    mid = rng.integers(0, 1 << (bits // 2), 9, dtype=np.uint64)[rng.integers(0, 9, n)]
+    return (top + mid + rng.integers(0, 200, n).astype(np.uint64)).astype(f"u{bits // 8}").view(dtype)
+
+
+@pytest.mark.parametrize("dtype", ["u4", "i4", "f4", "u8", "i8", "f8"])
+def test_keys_clustered_at_several_scales_match_oracle(ctx, orc, dtype):
+    """The sizes of one block, its edges and remainders, one and two levels of cells."""
+    block = {4: 512 * 20, 8: 512 * 14}[np.dtype(dtype).itemsize]
+    item = block // 512
+    rng = np.random.default_rng(8)
+    for n in (2, item - 1, item + 1, 2 * item, 33 * item + 5, block - 1, block, block + 1, 2 * block - item, 2 * block,
+              2 * block + 1, 100_003, 1 << 20, 5_000_011):
+        a = several_scales(dtype, n, rng)
+        assert sorted_on_device(ctx, a).tobytes() == orc.sort(a).tobytes(), f"{dtype} n={n}"
+
+
+@pytest.mark.parametrize("dtype,k", [("u4", 3), ("i4", 16), ("u8", 32), ("i8", 64)])
+def test_kway_tiles_of_integer_keys_match_oracle(ctx, orc, dtype, k):
+    """Merges whose tiles are sorted by bins: dense keys, clusters, one value; one key less and more than whole tiles."""
+    w = np.dtype(dtype).itemsize
+    tile = {4: 512 * 20, 8: 512 * 14}[w]
+    rng = np.random.default_rng(k)
+    for total in (k, tile - 1, tile, tile + 1, 5 * tile + 3):
+        for a in (several_scales(dtype, total, rng), rng.permutation(total).astype(f"u{w}").view(dtype),
+                  np.full(total, 9, dtype=dtype)):
+            cuts = np.sort(rng.integers(0, total + 1, k - 1))
+            runs = [orc.sort(r) if r.size else r for r in np.split(a, cuts)]
+            t = torch.from_numpy(np.concatenate(runs).view(np.int32 if w == 4 else np.int64).copy()).cuda()
+            out = torch.empty_like(t)
+            starts = np.concatenate([[0], cuts])
+            torch.cuda.synchronize()
+            ctx.kway_merge_device([t.data_ptr() + w * int(s) for s in starts], [r.size for r in runs], out.data_ptr(),
+                                  NAMES[dtype])
+            ctx.synchronize()
+            assert out.cpu().numpy().view(dtype).tobytes() == orc.sort(a).tobytes(), f"{dtype} k={k} total={total}"

@@ -2334,8 +2334,15 @@ cudaError_t launch_units(const Sort<B>& a, size_t max_units, unsigned sms, cudaS
   Sort<B> copy = a;
   u32 cur = a.last_list;
   void* args[] = {&copy, &cur};
+  // A cooperative grid starts when all its blocks can be resident. With 2 * sms blocks, all that fit, that was when
+  // the chip was empty, and kernels of other streams waited meanwhile: the serving loop on four streams came to 3.7
+  // Gkeys/s (requests of 2^10..2^18 keys) and 35 (2^10..2^26). With 64, 96, 128, 148, 222 or 256 blocks it came to
+  // 5.1-5.3 and 48-49; without this kernel the former to 5.5. A block per SM is also faster than two for the little
+  // that is mostly left (3 * 10^6 float64 heavy tail 249 / 280 us); from 2^24 keys on half as many more are (3.3 *
+  // 10^7 float32, a third zeros, infinities and NaN: 659 us with 148, 642 with 222; 5 * 10^7 in clusters 2.14 / 2.08 ms).
+  const unsigned tail_grid = a.n < (1u << 24) ? sms : sms + sms / 2;
   if (rec) rec->before("part_tail", stream);
-  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(tail), dim3(sms * 2), dim3(kThreads), args,
+  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(tail), dim3(tail_grid), dim3(kThreads), args,
                                   sizeof(TailSmem<B>), stream);
   if (rec) rec->after("part_tail", stream);
   return e;

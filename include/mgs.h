@@ -366,13 +366,15 @@ int mgs_generate_device(mgs_ctx* ctx, int dtype, const char* distribution, uint3
 /* ---- failure injection for tests (no counterpart in the reference, whose
  * CheckCudaError ignores errors in release builds, src/cuda_error.cuh:5-10) ----
  * mgs_test_set_waits: bounds of the sort kernels' device-side waits on
- * `device` (polls of a look-back status word, polls of a tile-copy barrier;
- * 0 = the default bound) for sorts launched afterwards, and one tile of the
- * plain device sort whose look-back status is never published (hold_tile;
- * 0xFFFFFFFF = none). With a tile held, the look-back after it waits on a word
- * that nothing sets until its bound runs out; the sort then finishes, its
- * output unspecified (every write stays inside the keys), and reports
- * MGS_ERR_TIMEOUT through mgs_ctx_synchronize. Call with (device, 0, 0,
+ * `device` (lookback_spins: polls of a look-back status word, and of the grid
+ * barrier of the partition sort's last kernel; tma_polls: polls of a tile-copy
+ * barrier; 0 = the default bound) for sorts launched afterwards, and one tile of
+ * the onesweep whose look-back status is never published (hold_tile;
+ * 0xFFFFFFFF = none; plain sorts run the onesweep while a tile is held). With a
+ * tile held, the look-back after it waits on a word that nothing sets until its
+ * bound runs out. A sort whose wait ran out finishes, its output unspecified
+ * (every write stays inside the keys), and reports MGS_ERR_TIMEOUT through
+ * mgs_ctx_synchronize. Call with (device, 0, 0,
  * 0xFFFFFFFF) to restore the defaults. Synchronous.
  * mgs_test_fail_device_allocations: the next `count` growths of any context's
  * device arena fail as an out-of-memory cudaMalloc would (MGS_ERR_OOM); 0

@@ -22,7 +22,7 @@
 //                       too large for it, cells that hold one value,
 //                       and, through the same steps once more, cells that two
 //                       levels left too large (keys clustered at several
-//                       scales); the zeros' signs; the status.
+//                       scales); the zeros' signs.
 // Inputs that one block can hold take a single launch (part_small).
 //
 // HBM traffic of one level: read + (read + write) + (read + write) = 5 n w;
@@ -337,7 +337,6 @@ struct State {
   u64 list[2];        // per segment list: segments << 32 | tiles
   u32 units, next_unit, left;
   u32 hist_done;
-  u32 error;
   u32 neg_zeros, pos_zeros, below_zeros;  // IEEE keys: -0.0, +0.0, keys that sort before them
   u32 barrier;
   u32 dirty;  // segments found to hold several values
@@ -443,15 +442,21 @@ __device__ __forceinline__ void block_min_max(B& lo, B& hi, B* mm) {
   hi = warp_max(in ? mm[32 + lane] : B(0));
 }
 
-// Blocks that wait on one another (cooperative launch): all arrive, bounded wait.
-__device__ __forceinline__ bool grid_barrier(State* st, u32 target) {
+// Polls of the grid barrier (set_barrier_spins).
+__device__ u32 g_barrier_spins = kBarrierSpins;
+
+// Blocks that wait on one another (cooperative launch): all arrive, bounded
+// wait. A block whose bound runs out reports it at once and must leave: the
+// others then cannot pass the next barrier, so no block works on a later step
+// than one past what every block has finished.
+__device__ __forceinline__ bool grid_barrier(State* st, u32 target, u32 spins, u32* status) {
   __shared__ u32 s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(&st->barrier, 1u);
     u32 ok = 0;
-    for (u32 i = 0; i < kBarrierSpins; ++i) {
+    for (u32 i = 0; i < spins; ++i) {
       if (ld_volatile_u32(&st->barrier) >= target) {
         ok = 1;
         break;
@@ -459,7 +464,7 @@ __device__ __forceinline__ bool grid_barrier(State* st, u32 target) {
       if (i > 16) __nanosleep(64);
     }
     __threadfence();
-    if (!ok) atomicOr(&st->error, kStatusQueueTimeout);
+    if (!ok && status != nullptr) atomicOr(status, kStatusQueueTimeout);
     s_ok = ok;
   }
   __syncthreads();
@@ -2094,13 +2099,14 @@ __device__ void probe_segments(const Sort<B>& a) {
 }
 
 // Cooperative launch. Sorts the units that are left, then goes on with the
-// segments of list `cur`, if any are left; last, the zeros' signs and the status.
+// segments of list `cur`, if any are left; last, the zeros' signs.
 template <typename B, int KIND>
 __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 cur) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   TailSmem<B>& sm = *reinterpret_cast<TailSmem<B>*>(smem_raw);
   __shared__ MapTable<B> tab;
   const u32 tid = threadIdx.x, G = gridDim.x, b = blockIdx.x;
+  const u32 spins = g_barrier_spins;
   u32 waits = 0;
   bool ok = true;
   constexpr int ITEMS = Shape<sizeof(B)>::kWideItems;
@@ -2112,7 +2118,7 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
   }
   if (__ldcg(&a.st->list[cur]) != 0u) {
     probe_segments<B, KIND>(a);
-    ok = grid_barrier(a.st, ++waits * G);
+    ok = grid_barrier(a.st, ++waits * G, spins, a.status);
   }
   // Probed segments of one value that sit in the caller's buffer: to the caller's bits. Tile by tile: a loop over the
   // segments in every block was a chain of dependent reads, 1.3 us per segment (27 segments, 3 * 10^6 float64 with a
@@ -2137,24 +2143,24 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
     const u32 t0 = u32(u64(tiles) * b / G), t1 = u32(u64(tiles) * (b + 1) / G);
     const u32 cells = nseg * 8u + tiles * kCellsPerTile<B>;
     for (u32 i = b * kThreads + tid; i < cells; i += G * kThreads) a.count0[i] = 0u;
-    if (!(ok = grid_barrier(a.st, ++waits * G))) break;
+    if (!(ok = grid_barrier(a.st, ++waits * G, spins, a.status))) break;
     if (b == 0 && tid == 0) {
       a.st->units = 0;
       a.st->list[cur ^ 1u] = 0;
     }
     map_segments<B, kUnsignedKey>(a, a.segs(cur), b, G, nseg, sm.map.map, sm.map.scratch);
-    if (!(ok = grid_barrier(a.st, ++waits * G))) break;
+    if (!(ok = grid_barrier(a.st, ++waits * G, spins, a.status))) break;
     histogram_tiles<B, kUnsignedKey, false>(a, a.segs(cur), nseg, a.count0, t0, t1, sm.hist);
-    if (!(ok = grid_barrier(a.st, ++waits * G))) break;
+    if (!(ok = grid_barrier(a.st, ++waits * G, spins, a.status))) break;
     for (u32 s = b; s < nseg; s += G) {
       if (__ldcg(&a.segs(cur)[s].done)) continue;
       __syncthreads();
       load_table<B>(tab, a.tables + s);
       plan_segment<B>(a, a.segs(cur) + s, load_map<B>(a.maps + s), tab, cur ^ 1u, false, false, a.count0, sm.plan);
     }
-    if (!(ok = grid_barrier(a.st, ++waits * G))) break;
+    if (!(ok = grid_barrier(a.st, ++waits * G, spins, a.status))) break;
     scatter_tiles<B, kUnsignedKey, false>(a, a.segs(cur), t0, t1, sm.scatter);
-    if (!(ok = grid_barrier(a.st, ++waits * G))) break;
+    if (!(ok = grid_barrier(a.st, ++waits * G, spins, a.status))) break;
     const u32 units = __ldcg(&a.st->units);
     for (u32 u = b; u < units; u += G) sort_any_unit<B, KIND, kThreads, ITEMS>(a, __ldcg(a.units + u), false, sm.local);
     const u32 more = __ldcg(&a.st->left);
@@ -2167,7 +2173,7 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
   if (KIND == kFloatKey && ok) {
     const u32 neg = __ldcg(&a.st->neg_zeros), pos = __ldcg(&a.st->pos_zeros);
     if (neg && !__ldcg(&a.st->in_place)) {
-      if ((waits || left) && !grid_barrier(a.st, ++waits * G)) return;  // every key is in its place
+      if ((waits || left) && !grid_barrier(a.st, ++waits * G, spins, a.status)) return;  // every key is in its place
       constexpr B sign = B(1) << (sizeof(B) * 8 - 1);
       const u32 lo = __ldcg(&a.st->below_zeros);
       const u32 zeros = neg + pos;
@@ -2175,10 +2181,6 @@ __global__ __launch_bounds__(kThreads, 2) void part_tail_kernel(Sort<B> a, u32 c
       for (u64 i = b * kThreads + tid; i < zeros; i += G * kThreads)  // 64 bits: a step past 2^32 must not wrap
         a.keys[lo + i] = !pos || ((__ldcg(a.zero_signs + (i >> 5)) >> (i & 31u)) & 1u) ? sign : B(0);
     }
-  }
-  if (b == 0 && tid == 0 && a.status != nullptr) {
-    const u32 error = __ldcg(&a.st->error);
-    if (error) atomicOr(a.status, error);
   }
 }
 
@@ -2444,6 +2446,11 @@ cudaError_t partition_segments(int dtype, void* d_keys, size_t n, const unsigned
                                                             rec);
   });
   return result;
+}
+
+cudaError_t set_barrier_spins(uint32_t spins) {
+  const u32 v = spins ? spins : kBarrierSpins;
+  return cudaMemcpyToSymbol(g_barrier_spins, &v, sizeof(v));
 }
 
 size_t kway_unit_tile_keys(int dtype) {

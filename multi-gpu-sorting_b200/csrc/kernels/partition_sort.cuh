@@ -19,6 +19,11 @@ size_t partition_sort_temp_bytes(int dtype, size_t n);
 cudaError_t partition_sort(int dtype, void* d_keys, size_t n, void* d_temp, size_t temp_bytes, cudaStream_t stream,
                            uint32_t* d_status, LaunchRecorder* rec);
 
+// Polls of the grid barrier of the sort's last kernel on the current device, for
+// sorts launched afterwards (0: the default). When they run out the kernel ends,
+// the keys are left unspecified and *d_status gets kStatusQueueTimeout.
+cudaError_t set_barrier_spins(uint32_t spins);
+
 // The large segments of a segmented sort of integer keys: segment ids[i], i <
 // *d_count <= max_segments, is [d_offsets[ids[i]], d_offsets[ids[i] + 1]) of
 // d_keys (all device arrays), of more than two blocks' worth of keys; each is

@@ -1951,7 +1951,8 @@ cudaError_t set_wait_control(uint32_t lookback_spins, uint32_t tma_polls, uint32
   const WaitControl wc{lookback_spins ? lookback_spins : kLookbackSpinLimit, tma_polls ? tma_polls : kTmaWaitLimit,
                        hold_tile, 0u};
   int dev = 0;
-  const cudaError_t e = cudaGetDevice(&dev);
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = set_barrier_spins(lookback_spins);
   if (e != cudaSuccess) return e;
   if (dev < 64) {
     const uint64_t bit = uint64_t(1) << dev;

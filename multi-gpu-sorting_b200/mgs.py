@@ -241,7 +241,8 @@ NO_HELD_TILE = 0xFFFFFFFF
 
 def inject_waits(device: int = 0, lookback_spins: int = 0, tma_polls: int = 0, hold_tile: int = NO_HELD_TILE):
     """mgs_test_set_waits (failure injection for tests): bounds of the device-side waits (0 = default) and a
-    tile of the plain device sort whose look-back status is never published. Defaults restore normal sorts."""
+    tile of the onesweep whose look-back status is never published (plain sorts run the onesweep while one is
+    held). Defaults restore normal sorts."""
     _check(load_library().mgs_test_set_waits(int(device), int(lookback_spins), int(tma_polls), int(hold_tile)))
 
 

@@ -210,3 +210,28 @@ def test_kway_tiles_of_integer_keys_match_oracle(ctx, orc, dtype, k):
                                   NAMES[dtype])
             ctx.synchronize()
             assert out.cpu().numpy().view(dtype).tobytes() == orc.sort(a).tobytes(), f"{dtype} k={k} total={total}"
+
+
+@pytest.mark.parametrize("dtype", ["u8", "i8", "f8"])
+def test_grid_barrier_that_runs_out_reports_timeout_and_context_recovers(mgs, orc, dtype):
+    """With a bound of one poll, the blocks that reach the last kernel's barrier before the others give up: the sort
+    ends with an error status, and the same context sorts again. The heavy value's cell makes the kernel probe its
+    keys, which ends at that barrier."""
+    a = heavy_end("ids", 1 << 20, np.random.default_rng(3)).view(dtype)
+    ctx = mgs.Context(0)
+    try:
+        t = torch.from_numpy(a.view(np.int64).copy()).cuda()
+        torch.cuda.synchronize()
+        mgs.inject_waits(0, lookback_spins=1)
+        try:
+            ctx.sort_device(t.data_ptr(), a.size, NAMES[dtype])
+            with pytest.raises(mgs.MgsError) as err:
+                ctx.synchronize()
+            assert err.value.code == mgs.MGS_ERR_TIMEOUT
+            assert "queue" in str(err.value)
+        finally:
+            mgs.inject_waits(0)
+        ctx.synchronize()  # the status was taken
+        assert sorted_on_device(ctx, a).tobytes() == orc.sort(a).tobytes()
+    finally:
+        ctx.close()

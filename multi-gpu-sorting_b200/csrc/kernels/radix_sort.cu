@@ -1586,8 +1586,9 @@ struct PairShape {
   static constexpr int kMinBlocks = 1, kChains = 1;
 };
 
+// shape: of a plain keys-only sort (the others have one shape each). The total does not depend on it.
 template <class Tr, typename V = NoValue, class Dg = PlainDigits>
-RadixLayout radix_layout(size_t n) {
+RadixLayout radix_layout(size_t n, int shape = kDefaultShape) {
   constexpr int w = int(sizeof(typename Tr::Bits));
   size_t tile;
   if constexpr (kHasValues<V>) {
@@ -1598,7 +1599,7 @@ RadixLayout radix_layout(size_t n) {
     constexpr size_t tiles[kNumShapes] = {shape_tile<w, 0>(), shape_tile<w, 1>(), shape_tile<w, 2>(),
                                            shape_tile<w, 3>(), shape_tile<w, 4>(), shape_tile<w, 5>(),
                                            shape_tile<w, 6>()};
-    tile = tiles[sort_variant(w, n).shape];
+    tile = tiles[shape];
   }
   // The look-back arrays are sized for the smallest tile, so every shape (and the key-value tiles) fits.
   constexpr size_t min_tile = shape_tile<w, 1>();
@@ -1659,7 +1660,7 @@ cudaError_t launch_onesweep_passes(typename Tr::Bits* keys, typename Tr::Bits* t
 
 template <class Tr, typename StatusT>
 cudaError_t launch_onesweep_variant(typename Tr::Bits* keys, typename Tr::Bits* tmp, RadixState* st, char* tbase,
-                                    const RadixLayout& L, uint32_t n, bool use_tma, cudaStream_t stream,
+                                    const RadixLayout& L, SortVariant v, uint32_t n, bool use_tma, cudaStream_t stream,
                                     LaunchRecorder* rec) {
 #define MGS_LAUNCH(S, M) launch_onesweep_passes<Tr, S, StatusT, M>(keys, tmp, st, tbase, L, n, use_tma, stream, rec)
 #define MGS_SHAPES(M)                \
@@ -1672,9 +1673,6 @@ cudaError_t launch_onesweep_variant(typename Tr::Bits* keys, typename Tr::Bits* 
     case 6: return MGS_LAUNCH(6, M); \
     default: return MGS_LAUNCH(5, M); \
   }
-  // The same choice as radix_layout made for this n (the table is read once per sort there and here;
-  // set_sort_variant must not run while sorts are being issued).
-  const SortVariant v = sort_variant(int(sizeof(typename Tr::Bits)), n);
   if (v.mode == 2) MGS_SHAPES(2)
   MGS_SHAPES(3)
 #undef MGS_SHAPES
@@ -1706,14 +1704,15 @@ cudaError_t launch_onesweep_pairs(typename Tr::Bits* keys, typename Tr::Bits* tm
   return cudaSuccess;
 }
 
-// Sorts keys (and, with a value type V, the values beside them) in place.
+// Sorts keys (and, with a value type V, the values beside them) in place. variant: of a plain keys-only sort.
 template <class Tr, typename V = NoValue, class Dg = PlainDigits>
 cudaError_t radix_sort_impl(typename Tr::Bits* keys, V* vals, size_t n, void* temp, size_t temp_bytes,
-                            cudaStream_t stream, uint32_t* d_status, LaunchRecorder* rec, Dg dg = Dg{}) {
+                            cudaStream_t stream, uint32_t* d_status, LaunchRecorder* rec, Dg dg = Dg{},
+                            SortVariant variant = SortVariant{kDefaultShape, kDefaultRankMode}) {
   using Bits = typename Tr::Bits;
   if (n == 0) return cudaSuccess;
   if (n >= (size_t(1) << 32)) return cudaErrorInvalidValue;
-  const RadixLayout L = radix_layout<Tr, V, Dg>(n);
+  const RadixLayout L = radix_layout<Tr, V, Dg>(n, variant.shape);
   if (temp == nullptr || temp_bytes < L.total) return cudaErrorInvalidValue;
   char* tb = static_cast<char*>(temp);
   RadixState* st = reinterpret_cast<RadixState*>(tb + L.state_off);
@@ -1763,21 +1762,14 @@ cudaError_t radix_sort_impl(typename Tr::Bits* keys, V* vals, size_t n, void* te
                                                                                  stream, rec, dg);
       }
     } else if (L.status_bytes == 4) {
-      e = launch_onesweep_variant<Tr, uint32_t>(keys, tmp, st, tb, L, n32, use_tma, stream, rec);
+      e = launch_onesweep_variant<Tr, uint32_t>(keys, tmp, st, tb, L, variant, n32, use_tma, stream, rec);
     } else {
-      e = launch_onesweep_variant<Tr, unsigned long long>(keys, tmp, st, tb, L, n32, use_tma, stream, rec);
+      e = launch_onesweep_variant<Tr, unsigned long long>(keys, tmp, st, tb, L, variant, n32, use_tma, stream, rec);
     }
     if (e != cudaSuccess) return e;
     return launch_kernel(rec, "radix_finalize", radix_finalize_kernel<Tr>, dim3(fin_grid), dim3(256), 0, stream, keys,
                          tmp, st, n32, d_status);
   }
-}
-
-template <class Tr>
-cudaError_t radix_sort_typed(typename Tr::Bits* keys, size_t n, void* temp, size_t temp_bytes, cudaStream_t stream,
-                             uint32_t* d_status, LaunchRecorder* rec) {
-  return radix_sort_impl<Tr, NoValue>(keys, static_cast<NoValue*>(nullptr), n, temp, temp_bytes, stream, d_status,
-                                      rec);
 }
 
 // ---------------------------------------------------------------- segmented host
@@ -2074,11 +2066,18 @@ cudaError_t segmented_sort(int dtype, void* d_keys, size_t n, const uint64_t* d_
 cudaError_t radix_sort(int dtype, void* d_keys, size_t n, void* d_temp, size_t temp_bytes, cudaStream_t stream,
                        uint32_t* d_status, LaunchRecorder* rec) {
   if (!onesweep_wanted(dtype, n)) return partition_sort(dtype, d_keys, n, d_temp, temp_bytes, stream, d_status, rec);
+  return onesweep_sort(dtype, d_keys, n, d_temp, temp_bytes, sort_variant(int(dtype_bytes(dtype)), n), stream, d_status,
+                       rec);
+}
+
+cudaError_t onesweep_sort(int dtype, void* d_keys, size_t n, void* d_temp, size_t temp_bytes, SortVariant v,
+                          cudaStream_t stream, uint32_t* d_status, LaunchRecorder* rec) {
   cudaError_t result = cudaErrorInvalidValue;
+  if (!valid_variant(v)) return result;
   dispatch_dtype(dtype, [&](auto tr) {
     using Tr = decltype(tr);
-    result = radix_sort_typed<Tr>(static_cast<typename Tr::Bits*>(d_keys), n, d_temp, temp_bytes, stream, d_status,
-                                  rec);
+    result = radix_sort_impl<Tr, NoValue>(static_cast<typename Tr::Bits*>(d_keys), static_cast<NoValue*>(nullptr), n,
+                                          d_temp, temp_bytes, stream, d_status, rec, PlainDigits{}, v);
   });
   return result;
 }

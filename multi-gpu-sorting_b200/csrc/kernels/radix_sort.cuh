@@ -94,6 +94,9 @@ bool valid_variant(SortVariant v);
 // false when out of range. pin: plain sorts of that class run this variant from then on (mgs_tune_set); without
 // it the entry is only what the table says, and plain sorts stay partition sorts (partition_sort.cuh).
 bool set_sort_variant(int key_bytes, int size_class, SortVariant v, bool pin);
+// The onesweep with a variant of the caller's choice, whatever the table says.
+cudaError_t onesweep_sort(int dtype, void* d_keys, size_t n, void* d_temp, size_t temp_bytes, SortVariant v,
+                          cudaStream_t stream, uint32_t* d_status, LaunchRecorder* rec);
 SortVariant sort_variant(int key_bytes, size_t n);  // the table's entry, then the environment overrides
 SortVariant table_variant(int key_bytes, int size_class);  // the table's entry alone
 // Tuning files (format in tune.cu): load returns the number of entries read,

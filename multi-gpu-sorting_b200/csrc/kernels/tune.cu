@@ -82,22 +82,16 @@ cudaError_t autotune(int dtype, size_t max_n, int reps, std::vector<TuneSample>*
     const size_t n = size_class_sample(c);
     if (n > max_n) continue;
     SortVariant best{-1, -1};
-    // Measured variants are pinned so that radix_sort runs them; whatever ends this class leaves none pinned.
-    struct Unpin {
-      int w, c;
-      ~Unpin() { set_sort_variant(w, c, table_variant(w, c), false); }
-    } unpin{int(w), c};
     double best_ms = 1e30;
     const size_t first = out ? out->size() : 0;
     for (int mode = 2; mode <= 3; ++mode) {
       for (int shape = 0; shape < 7; ++shape) {
         const SortVariant v{shape, mode};
-        if (!set_sort_variant(int(w), c, v, true)) continue;
         std::vector<float> t;
         for (int r = 0; r <= reps; ++r) {
           e = cudaMemcpyAsync(b.keys, b.pristine, n * w, cudaMemcpyDeviceToDevice, b.stream);
           if (e == cudaSuccess) e = cudaEventRecord(b.start, b.stream);
-          if (e == cudaSuccess) e = radix_sort(dtype, b.keys, n, b.temp, temp_bytes, b.stream, nullptr, nullptr);
+          if (e == cudaSuccess) e = onesweep_sort(dtype, b.keys, n, b.temp, temp_bytes, v, b.stream, nullptr, nullptr);
           if (e == cudaSuccess) e = cudaEventRecord(b.stop, b.stream);
           if (e == cudaSuccess) e = cudaEventSynchronize(b.stop);
           float ms = 0.f;

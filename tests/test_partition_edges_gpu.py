@@ -235,3 +235,22 @@ def test_grid_barrier_that_runs_out_reports_timeout_and_context_recovers(mgs, or
         assert sorted_on_device(ctx, a).tobytes() == orc.sort(a).tobytes()
     finally:
         ctx.close()
+
+
+def test_autotune_leaves_other_threads_sorts_alone(mgs, orc):
+    """The autotuner times onesweep variants; plain sorts that other threads issue meanwhile stay partition sorts."""
+    import threading
+    a = np.random.default_rng(4).integers(0, 1 << 32, 150_001, dtype=np.uint32)  # a size class that is being tuned
+    tuning, mine = mgs.Context(0), mgs.Context(0)
+    try:
+        mine.set_profiling(True)
+        th = threading.Thread(target=tuning.autotune, args=("u32", 3 << 16, 40))
+        th.start()
+        while th.is_alive():
+            assert sorted_on_device(mine, a).tobytes() == orc.sort(a).tobytes()
+        th.join()
+        names = set(mine.kernel_times())
+        assert "part_scatter" in names and "radix_onesweep" not in names
+    finally:
+        tuning.close()
+        mine.close()

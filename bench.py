@@ -1070,8 +1070,11 @@ def main():
         traffic = committed_traffic("part_scatter") if n == N_KEYS else None
         roof = {"bound": "hbm", "kernel": "part_scatter", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
-                "traffic": traffic, "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms}
-    sort_alg_bytes = 36 * n  # a radix sort's 4 passes x (read + write) + one histogram read, 4-byte keys
+                "traffic": traffic, "traffic_kind": "committed profile of 2^26 keys, scaled" if traffic else None,
+                "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms}
+    # Bytes the partition sort moves, 4-byte keys: per level a histogram's read and a scatter's read and write, then
+    # the block-local sorts' read and write; one level of cells up to 1022 * 3584 keys, two above.
+    sort_alg_bytes = (32 if n > 1022 * 3584 else 20) * n
     sort_ms = total_ms / args.steps
 
     batched = None

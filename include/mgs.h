@@ -101,7 +101,8 @@ int mgs_host_free(void* ptr);
  * bytes, or be NULL to use the context arena. stream is a cudaStream_t (NULL =
  * the context's compute stream). Asynchronous: device status is reported by
  * mgs_ctx_synchronize. n must be below 2^32. Runs a partition sort, unless
- * mgs_tune_set (or its environment variables) asked for an onesweep variant. */
+ * mgs_tune_set (or its environment variables) asked for an onesweep variant, or
+ * d_temp holds less than that, but what the onesweep needs. */
 int mgs_sort_temp_bytes(int dtype, size_t n, size_t* bytes);
 int mgs_sort_device(mgs_ctx* ctx, int dtype, void* d_keys, size_t n, void* d_temp, size_t temp_bytes,
                     void* stream);

@@ -98,9 +98,10 @@ void plan_release(mgs_plan* p) {
 
 // Records body(d_temp, temp_bytes, stream, recorder) into a graph on a private
 // stream (relaxed capture mode: the one-time per-kernel attribute calls the
-// launch path makes are allowed during the capture) and instantiates it.
+// launch path makes are allowed during the capture) and instantiates it. need:
+// the scratch it allocates itself; least: what it takes from the caller.
 template <class Body>
-int plan_record(mgs_ctx* ctx, const char* what, size_t need, void* d_temp, size_t temp_bytes, Body body,
+int plan_record(mgs_ctx* ctx, const char* what, size_t need, size_t least, void* d_temp, size_t temp_bytes, Body body,
                 mgs_plan** out) {
   Context& c = ctx->impl;
   DeviceGuard g(c.device);
@@ -120,7 +121,7 @@ int plan_record(mgs_ctx* ctx, const char* what, size_t need, void* d_temp, size_
     }
     d_temp = p->owned_temp;
     temp_bytes = need;
-  } else if (temp_bytes < need) {
+  } else if (temp_bytes < least) {
     plan_release(p);
     set_last_error("%s: d_temp holds %zu bytes, %zu needed", what, temp_bytes, need);
     return MGS_ERR_INVALID;
@@ -326,7 +327,7 @@ int mgs_sort_device(mgs_ctx* ctx, int dtype, void* d_keys, size_t n, void* d_tem
     if (e != cudaSuccess) return cuda_fail(e, "mgs_sort_device: arena");
     d_temp = c.arena;
     temp_bytes = c.arena_bytes;
-  } else if (temp_bytes < need) {
+  } else if (temp_bytes < mgs::onesweep_temp_bytes(dtype, n)) {
     set_last_error("mgs_sort_device: d_temp holds %zu bytes, %zu needed", temp_bytes, need);
     return MGS_ERR_INVALID;
   }
@@ -424,7 +425,7 @@ int mgs_sort_range_device(mgs_ctx* ctx, int dtype, void* d_keys, void* d_values,
   Context& c = ctx->impl;
   DeviceGuard g(c.device);
   const size_t need =
-      value_bytes ? mgs::radix_sort_pairs_temp_bytes(dtype, value_bytes, n) : mgs::radix_sort_temp_bytes(dtype, n);
+      value_bytes ? mgs::radix_sort_pairs_temp_bytes(dtype, value_bytes, n) : mgs::onesweep_temp_bytes(dtype, n);
   if (d_temp == nullptr) {
     cudaError_t e = c.reserve(need);
     if (e != cudaSuccess) return cuda_fail(e, "mgs_sort_range_device: arena");
@@ -679,7 +680,7 @@ int mgs_plan_sort_create(mgs_ctx* ctx, int dtype, void* d_keys, size_t n, void* 
   if (reinterpret_cast<uintptr_t>(d_keys) % w != 0) return invalid("mgs_plan_sort_create: d_keys is not key-aligned");
   if (n > kMaxDeviceSortKeys) return invalid("mgs_plan_sort_create: n must be below 2^32");
   const size_t need = n ? mgs::radix_sort_temp_bytes(dtype, n) : 0;
-  return plan_record(ctx, "mgs_plan_sort_create", need, d_temp, temp_bytes,
+  return plan_record(ctx, "mgs_plan_sort_create", need, n ? mgs::onesweep_temp_bytes(dtype, n) : 0, d_temp, temp_bytes,
                      [&](void* t, size_t tb, cudaStream_t s, mgs::LaunchRecorder* rec) {
                        return mgs::radix_sort(dtype, d_keys, n, t, tb, s, ctx->impl.d_status, rec);
                      },
@@ -699,7 +700,7 @@ int mgs_plan_segmented_create(mgs_ctx* ctx, int dtype, void* d_keys, size_t n, c
   if (n > kMaxDeviceSortKeys || num_segments >= kMaxDeviceSortKeys)
     return invalid("mgs_plan_segmented_create: n and num_segments must be below 2^32");
   const size_t need = empty ? 0 : mgs::segmented_sort_temp_bytes(dtype, n, num_segments);
-  return plan_record(ctx, "mgs_plan_segmented_create", need, d_temp, temp_bytes,
+  return plan_record(ctx, "mgs_plan_segmented_create", need, need, d_temp, temp_bytes,
                      [&](void* t, size_t tb, cudaStream_t s, mgs::LaunchRecorder* rec) {
                        if (empty) return cudaSuccess;
                        return mgs::segmented_sort(dtype, d_keys, n, d_offsets, num_segments, t, tb, s,

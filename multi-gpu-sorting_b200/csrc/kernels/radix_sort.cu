@@ -1957,10 +1957,14 @@ cudaError_t set_wait_control(uint32_t lookback_spins, uint32_t tma_polls, uint32
   return cudaMemcpyToSymbol(g_wait_control, &wc, sizeof(wc));
 }
 
-size_t radix_sort_temp_bytes(int dtype, size_t n) {
+size_t onesweep_temp_bytes(int dtype, size_t n) {
   size_t bytes = 0;
   dispatch_dtype(dtype, [&](auto tr) { bytes = radix_layout<decltype(tr)>(n).total; });
-  return std::max(bytes, partition_sort_temp_bytes(dtype, n));  // either path may run (radix_sort)
+  return bytes;
+}
+
+size_t radix_sort_temp_bytes(int dtype, size_t n) {
+  return std::max(onesweep_temp_bytes(dtype, n), partition_sort_temp_bytes(dtype, n));  // either may run (radix_sort)
 }
 
 size_t radix_sort_pairs_temp_bytes(int dtype, size_t value_bytes, size_t n) {
@@ -2065,7 +2069,8 @@ cudaError_t segmented_sort(int dtype, void* d_keys, size_t n, const uint64_t* d_
 
 cudaError_t radix_sort(int dtype, void* d_keys, size_t n, void* d_temp, size_t temp_bytes, cudaStream_t stream,
                        uint32_t* d_status, LaunchRecorder* rec) {
-  if (!onesweep_wanted(dtype, n)) return partition_sort(dtype, d_keys, n, d_temp, temp_bytes, stream, d_status, rec);
+  if (!onesweep_wanted(dtype, n) && temp_bytes >= partition_sort_temp_bytes(dtype, n))
+    return partition_sort(dtype, d_keys, n, d_temp, temp_bytes, stream, d_status, rec);
   return onesweep_sort(dtype, d_keys, n, d_temp, temp_bytes, sort_variant(int(dtype_bytes(dtype)), n), stream, d_status,
                        rec);
 }

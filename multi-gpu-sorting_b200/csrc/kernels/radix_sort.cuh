@@ -23,9 +23,13 @@ cudaError_t set_wait_control(uint32_t lookback_spins, uint32_t tma_polls, uint32
 // Bytes of scratch memory (device) one sort of n keys of the given dtype needs:
 // the ping-pong key buffer, the per-sort state block and two look-back arrays.
 size_t radix_sort_temp_bytes(int dtype, size_t n);
+// The least that radix_sort takes, at most radix_sort_temp_bytes: with less than the partition sort needs it runs the
+// onesweep. Range sorts of keys alone always do.
+size_t onesweep_temp_bytes(int dtype, size_t n);
 
 // Sorts d_keys[0..n) ascending and stably, in place, on `stream`. d_temp must
-// hold radix_sort_temp_bytes(dtype, n) bytes. Device-side failures (a bounded
+// hold onesweep_temp_bytes(dtype, n) bytes; with radix_sort_temp_bytes it may
+// run the partition sort, which is faster. Device-side failures (a bounded
 // wait that gave up) are OR-ed into *d_status (a device word) when it is not
 // null. Asynchronous.
 cudaError_t radix_sort(int dtype, void* d_keys, size_t n, void* d_temp, size_t temp_bytes, cudaStream_t stream,

@@ -254,3 +254,41 @@ def test_autotune_leaves_other_threads_sorts_alone(mgs, orc):
     finally:
         tuning.close()
         mine.close()
+
+
+@pytest.mark.parametrize("dtype", ["u4", "f4", "u8", "f8"])
+def test_scratch_of_the_onesweep_is_enough(ctx, mgs, orc, dtype):
+    """The partition sort needs more scratch than the onesweep at many sizes. Scratch that holds only the onesweep's
+    state, look-back words and second buffer is still taken, by plain, recorded and range sorts; a byte less is not."""
+    name, w = NAMES[dtype], np.dtype(dtype).itemsize
+    up = lambda x: (x + 255) // 256 * 256
+    rng = np.random.default_rng(9)
+    for n in (30_000, 100_000, 1 << 20):
+        tile = {4: 4096, 8: 2048}[w]
+        least = 16640 + 2 * up((n + tile - 1) // tile * 1024) + up(n * w)
+        assert least < ctx.sort_temp_bytes(name, n)
+        a = rng.integers(0, 1 << 31, n).astype(f"u{w}").view(dtype)
+        temp = torch.full((least + 4096,), 0x5A, dtype=torch.uint8, device="cuda")
+        t = torch.empty(n, dtype=torch.int32 if w == 4 else torch.int64, device="cuda")
+        keys, want = torch.from_numpy(a.view(np.int32 if w == 4 else np.int64).copy()).cuda(), orc.sort(a).tobytes()
+
+        def check(sort):
+            t.copy_(keys)
+            torch.cuda.synchronize()
+            sort()
+            ctx.synchronize()
+            assert t.cpu().numpy().tobytes() == want
+            assert bool((temp[least:] == 0x5A).all())
+
+        check(lambda: ctx.sort_device(t.data_ptr(), n, name, temp.data_ptr(), least))
+        check(lambda: ctx.sort_range_device(t.data_ptr(), n, name, 0, 8 * w, False, 0, 0, temp.data_ptr(), least))
+        plan = ctx.plan_sort(t.data_ptr(), n, name, temp.data_ptr(), least)
+        try:
+            check(plan.launch)
+        finally:
+            plan.close()
+        for refused in (lambda: ctx.sort_device(t.data_ptr(), n, name, temp.data_ptr(), least - 1),
+                        lambda: ctx.plan_sort(t.data_ptr(), n, name, temp.data_ptr(), least - 1)):
+            with pytest.raises(mgs.MgsError) as err:
+                refused()
+            assert err.value.code == mgs.MGS_ERR_INVALID
